@@ -27,6 +27,7 @@ struct g3x_ctx {
     int cls_timed[g3x::kMaxBuckets];        // 1 when the last batch recorded class k
     int64_t step_limit;                     // g3x_set_step_limit (0: the kernels' own bound)
     int no_int16;                           // g3x_set_int16(ctx, 0): width classes in int32 only
+    int tiles_set;                          // width classes given by g3x_set_tiles
 };
 
 namespace g3x {
@@ -261,6 +262,61 @@ static int launch_classes(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParam
     return rc;
 }
 
+// The group-per-job kernel or the width classes.  A lane class lasts as long as its longest job
+// (0.5-1.1 ms at 250 bases, whatever its job count) and then costs 5.5-8 ns a job; a group costs
+// 17-23 ns a job and 0.1 ms at least.  Measured on batches of uneven left and right extensions, group
+// against lanes: 62 jobs 113 and 606 us, 9.9k jobs 290 and 1107, 19.8k 403 and 1041, 39.6k 709 and
+// 1148, 79k 1343 and 1108; right extensions of 1-150 bases: 20k 504 and 960, 40k 925 and 973; w = 30:
+// 19.8k 344 and 541, 39.6k 592 and 579.  So batches up to 32k jobs take the groups.  A seed call
+// (left wave, right wave and their retry waves) pays the lanes' latency more often: 20k seeds 904 and
+// 2319 us, 40k 1520 and 2379, 80k 2814 and 2360, so its waves take them up to 48k.  Waves that run
+// side by side (the seed stream's) fill the lanes together and count together.
+constexpr int64_t kGroupJobs = 32768, kGroupSeeds = 49152;
+// Up to here a job takes a warp in the order given: 62 jobs 113 us against 126 sorted into classes
+// (three launches less), 2k 190 against 216, 4k 249 against 264 and, for the shorter right
+// extensions, 5k 295 against 248.
+constexpr int64_t kDirectJobs = 3072;
+
+// Contexts with width classes of their own (g3x_set_tiles), in int32 or with class timing keep to
+// them.
+static bool groups_allowed(const g3x_ctx* ctx) { return !ctx->tiles_set && !ctx->no_int16 && !ctx->timing; }
+
+// Runs a batch (or with base.order a wave of at most base.n jobs) through the group-per-job
+// kernel: up to kDirectJobs jobs as they are listed, a warp each; beyond, sorted into the
+// kernel's classes, up to eight jobs a warp.  The jobs it cannot take follow in the row-parallel
+// kernel.
+static int run_grouped(const LaunchDesc& base, const ScoreParams& sp, SchedScratch& s, int32_t* queue,
+                       cudaStream_t st) {
+    const bool direct = base.n <= kDirectJobs;
+    LaunchDesc rest = base;
+    int rc;
+    if (cudaMemsetAsync(queue, 0, kQueueInts * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
+    LaunchDesc d = base;
+    d.queue = queue;
+    if (direct) {
+        rc = launch_group16(d, sp, s.order, queue + 9, st);
+        rest.order_off = nullptr;
+        rest.count = queue + 9;
+    } else {
+        TileTable tt;
+        group16_tiles(tt);
+        if ((rc = schedule_jobs(s, base.jobs, base.n, sp, nullptr, tt, st, base.order, base.count))) return rc;
+        d.order = s.order;
+        d.order_off = s.bucket_oc;
+        rc = launch_group16(d, sp, nullptr, nullptr, st);
+        rest.order_off = s.bucket_oc + 2 * (tt.n - 1);
+        rest.count = rest.order_off + 1;
+    }
+    if (rc) return rc;
+    rest.order = s.order;
+    rest.queue = queue + 8;
+    rest.kernel = kKernelRowpar;
+    rest.lanes = 32; rest.tile = 9; rest.warp_batch = 0; rest.refill = 1;
+    rest.persistent = 1; rest.warps_per_block = 4;
+    rest.pdl = !direct;
+    return launch_rowpar(rest, sp, st);
+}
+
 // Schedules and runs a persistent batch: cost per job (length, or the model's prediction),
 // counting sort into width classes, one launch per class.
 static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams& sp, bool learned,
@@ -268,6 +324,12 @@ static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams
     int rc = alloc_sched(ctx->sched, base.n);
     if (rc) return rc;
     if (learned && (!ctx->model.params || !ctx->model.trained)) return G3X_ERR_NOT_TRAINED;
+    if (groups_allowed(ctx) && base.n <= kGroupJobs) {
+        LaunchDesc d = base;
+        d.stats = ctx->d_stats;
+        if (cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), st) != cudaSuccess) return G3X_ERR_CUDA;
+        return run_grouped(d, sp, ctx->sched, ctx->d_queue, st);
+    }
     rc = learned && ctx->model.active
              ? schedule_jobs_learned(ctx->sched, base.jobs, base.n, base.codes, base.nmask, base.n_bases,
                                      ctx->model.params, sp, ctx->tiles, st)
@@ -284,6 +346,10 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     g3x_ctx* ctx = w->ctx;
     const ClassRes res = w->res ? *w->res : ctx_res(ctx);
     SchedScratch& sched = *res.sched;
+    // A retry wave holds the few jobs whose band was too narrow (their count stays on the device):
+    // in groups it lasts 0.1 ms where a lane class of a handful of jobs lasts 0.5.
+    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= kGroupSeeds))
+        return run_grouped(d, sp, sched, res.queue, st);
     int rc = w->learned && ctx->model.active
                  ? schedule_jobs_learned(sched, d.jobs, d.n, d.codes, d.nmask, d.n_bases, ctx->model.params, sp,
                                          ctx->tiles, st, d.order, d.count)
@@ -309,6 +375,7 @@ static int seed_waves(g3x_ctx* ctx, const g3x_batch_opts_t* opts, const LaunchDe
     cw->ctx = ctx;
     cw->learned = learned;
     cw->res = nullptr;
+    cw->at_once = 1;
     wr->run = run_class_wave;
     wr->user = cw;
     *out = wr;
@@ -501,6 +568,7 @@ int g3x_set_tiles(g3x_ctx* ctx, const g3x_tile_t* h, int32_t n) {
             (lane && (t.refill < 1 || t.refill > 32)))
             return G3X_ERR_INVALID;
     }
+    ctx->tiles_set = 1;
     ctx->tiles.n = n;
     for (int k = 0; k < n; ++k) {
         ctx->tiles.width[k] = k == n - 1 ? 0x7FFFFFFF : h[k].width;

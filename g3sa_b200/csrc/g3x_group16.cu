@@ -1,0 +1,424 @@
+// g3x_group16.cu -- group-per-job sm_100a kernel for batched ksw_extend2 in int16x2
+// (bwa/src/ksw.cu:303-401), for batches too small to fill the lane-per-job kernel.
+//
+// The lane-per-job kernel (g3x_lane16.cu) needs tens of thousands of jobs: a lane walks its row
+// block by block, 2,000-3,400 cycles a row for 200 columns, so a batch lasts as long as its
+// longest job (0.5-0.6 ms at 250 bases) however few jobs it has.  Here a group of G lanes runs a
+// job and a row is one step: lane r of the group holds columns 8r .. 8r + 7 of the row buffer
+// (ksw.cu:310) in registers for the whole job, as the same four int16x2 words of H and four of E
+// per eight-column block (word p = columns 8r + p and 8r + p + 4), with the block's query codes
+// beside them.  G = 4, 8, 16 or 32 by query length (up to 31, 63, 127, 255 bases: the group
+// holds column qlen too), so a warp runs 8 to 1 jobs.  Nothing of a row touches memory.
+//
+// One row: every lane runs the block recurrence of g3x_lane16.cuh; the F that enters each block
+// is a max-plus prefix over the group (log2 G shuffles of the blocks' outgoing F, decaying by
+// 8 e_ins per lane); H of the column left of a block comes from the lane before it by one
+// shuffle; the row maximum with its last column is one max over (H << 16 | column) keys; and the
+// band trims (ksw.cu:388-391) take the first and last lane of a ballot over the lanes' non-zero
+// column masks.  Band edges follow g3x_lane16.cuh: columns left of beg hold zeros (the words the
+// band clamp cuts off are zeroed), columns right of end keep their words, column end gets
+// {H(i, end-1), 0}, which the shifted H words of its block hold already.
+//
+// What bounds it: latency for small batches (a row is one dependent chain of about 300 cycles,
+// half of it the shuffles of the F prefix), issue slots (about 150 instructions a warp row)
+// beyond a few thousand jobs.
+#include <cuda_runtime.h>
+#include "g3x_core.h"
+#include "g3x_internal.h"
+#include "g3x_lane16.cuh"
+#include "g3x_stage.cuh"
+
+namespace g3x {
+
+namespace {
+
+using namespace l16;
+
+constexpr unsigned kAll = 0xFFFFFFFFu;
+constexpr int kBlockWarps = 2;
+
+// Masks by h = clamp(end - first column of the block, -1, 8), entry h + 1: the pair words of
+// the columns left of end and right of end, and the bits of the columns up to end.
+struct EdgeTable {
+    uint4 left[10], right[10];
+    uint32_t upto[10];
+};
+
+// A decay of `steps` lanes for values held in the high half of a word; values stay below 2^15,
+// so a decay of 2^15 - 1 already leaves nothing.
+__device__ __forceinline__ int32_t decay_hi(int32_t e_ins, int steps) {
+    const int32_t v = 8 * steps * e_ins;
+    return -((v < 0x7FFF ? v : 0x7FFF) << 16);
+}
+
+// No row yet: below every row's key but those of rows without a positive cell (columns stay below
+// 256).
+constexpr int32_t kNoRow = 0xFFFF;
+constexpr int32_t kNoGscore = -2;   // no to-end score in a row: below gscore's start
+
+// Largest of the group's values, in every lane of it.
+template <int G>
+__device__ __forceinline__ int32_t max_of_group(int32_t v) {
+    if constexpr (G == 32) {
+        return __reduce_max_sync(kAll, v);
+    } else {
+#pragma unroll
+        for (int o = G / 2; o >= 1; o >>= 1) v = max(v, __shfl_xor_sync(kAll, v, o));
+        return v;
+    }
+}
+
+// Exclusive prefix over the lanes of a group of the F leaving each block (high halves of x): F
+// entering the lane's block, where a value loses 8 e_ins per lane it passes.  A lane that a
+// shuffle leaves alone meets its own value, less the decay.  For G = 32, where a row's latency
+// counts, three lanes per step (four dependent shuffles instead of six).
+template <int G>
+__device__ __forceinline__ int32_t f_entering(int32_t x, int r, int32_t e_ins) {
+    const int32_t y = __shfl_up_sync(kAll, x, 1, G);
+    int32_t f = r ? y : 0;
+    if constexpr (G < 32) {
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) f = __viaddmax_s32(__shfl_up_sync(kAll, f, o, G), decay_hi(e_ins, o), f);
+    } else {
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 2) {
+            const int32_t a = __shfl_up_sync(kAll, f, o), b = __shfl_up_sync(kAll, f, 2 * o);
+            const int32_t c = __shfl_up_sync(kAll, f, 3 * o);
+            f = __viaddmax_s32(a, decay_hi(e_ins, o), f);
+            f = __viaddmax_s32(b, decay_hi(e_ins, 2 * o), f);
+            f = __viaddmax_s32(c, decay_hi(e_ins, 3 * o), f);
+        }
+        f = __viaddmax_s32(__shfl_up_sync(kAll, f, 16), decay_hi(e_ins, 16), f);
+    }
+    return f;
+}
+
+// v >> n for any n as an unsigned shift amount: 0 from 32 on.
+__device__ __forceinline__ uint32_t shr_clamp(uint32_t v, uint32_t n) {
+    uint32_t r;
+    asm("shr.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+    return r;
+}
+
+// One group's job (uniform over its lanes, but for gscore and max_ie, which count only in the
+// lane that holds column qlen).
+struct GroupJob {
+    int32_t job;                   // -1: none
+    int32_t qlen, tlen, w;
+    int32_t i;                     // the next row
+    int32_t hv;                    // h0 - o_del - e_del (i + 1)
+    uint32_t t_off;
+    bool trev;
+    int32_t best, best_i, best_d;  // the maximum, its row, its diagonal (row - column)
+    int32_t max_off, gscore, max_ie, cells;
+    uint32_t qsel;                 // prmt selector of column qlen's H from words 0-1 or 2-3
+};
+
+// Runs the jobs order[0 .. n) (order null: 0 .. n) of one class with groups of G lanes, taken from
+// *queue.  misfit non-null: jobs that do not fit (query, int16) go to misfit[0 .. *misfits)
+// instead of being refused.
+//
+// The row loop is rotated so that the parts of a row that only decide (its maximum, z-drop, the
+// next band) overlap the next row's blocks, whose inputs they are not: an iteration starts with
+// row i's blocks and F prefix, then finishes row i - 1's bookkeeping from the reductions issued at
+// its end, and then completes row i within the band that this gives.
+template <int G, bool kSym>
+__device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParams& sp, const PairConst& pc,
+                                           const EdgeTable& tab, const uint2* pools, const int32_t* order, int n,
+                                           int32_t* queue, int32_t* misfit, int32_t* misfits, int lane,
+                                           unsigned long long& busy, unsigned long long& idle,
+                                           unsigned long long& waves) {
+    constexpr int kGroups = 32 / G;
+    const int r = lane & (G - 1), gb = lane & ~(G - 1);
+    const unsigned gmask = (G == 32 ? kAll : ((1u << G) - 1u)) << gb;
+    unsigned leaders = 0;
+#pragma unroll
+    for (int k = 0; k < kGroups; ++k) leaders |= 1u << (k * G);
+    const int col0 = 8 * r;
+    const int32_t zdrop = sp.zdrop > 0 ? sp.zdrop : 0x7FFFFFFF;
+
+    GroupJob J = {};
+    J.job = -1;
+    uint32_t H[4] = {0u, 0u, 0u, 0u}, E[4] = {0u, 0u, 0u, 0u};
+    uint32_t qw = 0, tw = 0;      // query codes of the block; target codes of rows 8 (r + G c) ..
+    uint2 pl = pools[0];          // score pools of row i
+    // row i - 1: (maximum << 16 | its last column), its to-end score, its band, and its first and
+    // last lanes with non-zero columns with their masks
+    int32_t key = kNoRow, gval = kNoGscore, end = 0;
+    int fl = 0, ll = 0;
+    uint32_t nzf = 1u, nzl = 1u;
+    bool exhausted = false, all_idle = true;
+    int32_t iters = 0;
+    unsigned long long rows = 0;
+    for (;;) {
+        // ---- row i: the blocks with F from zero, and the F entering each ----
+        RowState rs;
+        rs.plo = pl.x; rs.phi = pl.y;
+        BlockA a;
+        uint32_t ne[4], nh[4], h2[4];
+        phase_a<kSym>(H, E, qw, rs, pc, a, ne);
+        rs.fr = (uint32_t)f_entering<G>((int32_t)__viaddmax_s16x2(a.L2[3] << 16, pc.n4, a.L2[3]), r, sp.e_ins);
+        rs.hlast = 0u;
+        // score pools of row i + 1: lane r holds the target codes of rows i0 + 8r .. + 7, i0 the
+        // last multiple of 8 G rows
+        const int32_t i1 = J.i + 1;
+        if ((i1 & (8 * G - 1)) == 0) {
+            const int ch = (i1 >> 4) + (r >> 1);
+            if (ch << 4 < J.tlen) {
+                uint32_t x, nb;
+                load16(d.codes, d.nmask, J.t_off, J.tlen, ch, J.trev, x, nb);
+                tw = (uint32_t)(nibbles16(x, nb) >> ((r & 1) << 5));
+            }
+        }
+        // (the funnel shift takes its amount modulo 32)
+        const uint32_t t8 = __shfl_sync(kAll, tw, gb | ((i1 >> 3) & (G - 1)));
+        pl = pools[__funnelshift_r(t8, 0u, i1 << 2) & 7u];
+
+        // ---- row i - 1's bookkeeping (ksw.cu:371-386) ----
+        J.max_ie = gval >= J.gscore ? J.i - 1 : J.max_ie;
+        J.gscore = max(J.gscore, gval);
+        const int32_t m = key >> 16, dg = J.i - 1 - (key & 0xFFFF);
+        const bool up = m > J.best;
+        // z-drop: best - m, less the gap between the diagonals (never for a new maximum)
+        const int32_t t = dg - J.best_d;
+        const bool zstop = J.best - m - max(t * sp.e_del, -t * sp.e_ins) > zdrop;
+        J.max_off = max(J.max_off, up ? abs(dg) : 0);
+        J.best = max(J.best, m);
+        J.best_i = up ? J.i - 1 : J.best_i;
+        J.best_d = up ? dg : J.best_d;
+        // no positive cell, z-drop or the last row; or no job in any group
+        const bool stop = J.job >= 0 ? (uint32_t)key < (uint32_t)kNoRow || zstop || J.i >= J.tlen : all_idle;
+        if (__any_sync(kAll, stop)) {
+            const int owner = gb + (J.qlen >> 3);             // holds column qlen
+            const int32_t gs = __shfl_sync(kAll, J.gscore, owner & 31), gi = __shfl_sync(kAll, J.max_ie, owner & 31);
+            if (stop && J.job >= 0) {
+                if (r == 0) {
+                    d.out[J.job] = g3x_ext_t{J.best, J.best_i - J.best_d + 1, J.best_i + 1, gi + 1, gs, J.max_off};
+                    d.status[J.job] = G3X_OK;
+                    if (d.cells) d.cells[J.job] = J.cells;
+                    if (d.rows) d.rows[J.job] = J.i;
+                    rows += J.i;
+                }
+                J.job = -1;
+                J.tlen = 0;                                    // no more target codes to load
+            }
+            // refill together once half of the groups are idle: a refill waits for two dependent
+            // global loads, and jobs of a class and length come one after another
+            const unsigned idle = __ballot_sync(kAll, J.job < 0);
+            if (exhausted ? idle == kAll : 2 * __popc(idle) >= 32) {
+                if (exhausted) break;
+                const unsigned want = idle & leaders;
+                int first = 0;
+                if (lane == 0) first = atomicAdd(queue, __popc(want));
+                first = __shfl_sync(kAll, first, 0);
+                exhausted = first + __popc(want) >= n;
+                ++waves;
+                const int slot = first + __popc(want & ((1u << gb) - 1u));
+                bool fresh = false;
+                if (J.job < 0 && slot < n) {
+                    const int job = order ? order[slot] : slot;
+                    const g3x_job_t jb = d.jobs[job];
+                    JobConst c;
+                    c.qlen = jb.qlen; c.tlen = jb.tlen; c.h0 = jb.h0;
+                    c.o_del = sp.o_del; c.e_del = sp.e_del; c.o_ins = sp.o_ins; c.e_ins = sp.e_ins;
+                    c.oe_del = sp.oe_del; c.oe_ins = sp.oe_ins; c.zdrop = sp.zdrop;
+                    c.w = clamp_w(jb.w, c.qlen, sp.max_sc, sp.end_bonus, sp.o_del, sp.e_del, sp.o_ins, sp.e_ins);
+                    const bool fits = c.qlen < 8 * G && job_fits_int16(c, sp.max_sc);
+                    const bool too_long = c.qlen > d.qmax || c.tlen > d.tmax || !fits;
+                    const bool outside = !job_in_planes(jb, d.n_bases);
+                    if (!fits && misfit) {
+                        if (r == 0) misfit[atomicAdd(misfits, 1)] = job;
+                    } else if (too_long || outside || c.tlen == 0) {
+                        // refused before any base is read, or no rows: the initial results
+                        if (r == 0) {
+                            d.out[job] = too_long || outside ? g3x_ext_t{0, 0, 0, 0, 0, 0}
+                                                             : g3x_ext_t{c.h0, 0, 0, 0, -1, 0};
+                            d.status[job] = too_long ? G3X_ERR_TOO_LONG : outside ? G3X_ERR_INVALID : G3X_OK;
+                            if (d.cells) d.cells[job] = 0;
+                            if (d.rows) d.rows[job] = 0;
+                        }
+                    } else {
+                        fresh = true;
+                        J.job = job;
+                        J.qlen = c.qlen; J.tlen = c.tlen; J.w = c.w;
+                        J.i = 0;
+                        J.hv = c.h0 - c.oe_del;
+                        J.t_off = jb.t_off;
+                        J.trev = (jb.flags & G3X_JOB_TREV) != 0;
+                        J.best = c.h0; J.best_i = J.gscore = J.max_ie = -1;
+                        J.best_d = J.max_off = J.cells = 0;
+                        // column t of a block: half t >> 2 of word t & 3
+                        const uint32_t b2 = ((c.qlen & 1) ? 0x54u : 0x10u) + ((c.qlen & 4) ? 0x22u : 0u);
+                        J.qsel = b2 | (8u | b2 >> 4) * 0x1100u;      // zero-extended by H's sign
+                        // the block's query codes and the first rows' target codes: halves of
+                        // 16-base chunks
+                        const int c0 = (r >> 1) << 4, half = (r & 1) << 5;
+                        uint32_t x, nb;
+                        qw = tw = 0;
+                        if (c0 < c.qlen) {
+                            load16(d.codes, d.nmask, jb.q_off, c.qlen, r >> 1, (jb.flags & G3X_JOB_QREV) != 0, x, nb);
+                            qw = (uint32_t)(nibbles16(x, nb) >> half);
+                        }
+                        if (c0 < c.tlen) {
+                            load16(d.codes, d.nmask, J.t_off, c.tlen, r >> 1, J.trev, x, nb);
+                            tw = (uint32_t)(nibbles16(x, nb) >> half);
+                        }
+                        // row -1 (ksw.cu:317-319)
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            const int j = col0 + p;
+                            const uint32_t lo = j <= c.qlen + 1 ? (uint32_t)init_h(j, c) : 0u;
+                            const uint32_t hi = j + 4 <= c.qlen + 1 ? (uint32_t)init_h(j + 4, c) : 0u;
+                            H[p] = (lo & 0xFFFFu) | (hi << 16);
+                            E[p] = 0u;
+                        }
+                        // the band of row 0: all of [0, qlen)
+                        fl = gb; nzf = 1u;
+                        ll = gb + 64; nzl = 1u;
+                        end = c.qlen;
+                    }
+                }
+                // start the iteration anew: nothing is left of row i - 1, and a new job's blocks
+                // are still to come
+                const uint32_t t0 = __shfl_sync(kAll, tw, gb);
+                pl = fresh ? pools[t0 & 7u] : make_uint2(rs.plo, rs.phi);
+                all_idle = __all_sync(kAll, J.job < 0);
+                key = J.best << 16 | kNoRow;
+                gval = kNoGscore;
+                continue;
+            }
+        }
+        ++iters;
+
+        // ---- the band of row i (ksw.cu:388-391, then 335-345) ----
+        const int32_t cut = J.i - J.w;
+        const int32_t beg = max(8 * (fl - gb) + ffs32(nzf) - 1, cut);
+        end = min(min(8 * (ll - gb) + msb32(nzl) + 2, J.i + J.w + 1), J.qlen);
+        const int32_t h1 = beg == 0 ? max(J.hv, 0) : 0;
+        J.hv -= sp.e_del;
+        J.cells += max(end - beg, 0);
+        const int h = max(min(end - col0, 8), -1) + 1;
+        const uint4 lv = tab.left[h], rv = tab.right[h];
+        const uint32_t left[4] = {lv.x, lv.y, lv.z, lv.w}, right[4] = {rv.x, rv.y, rv.z, rv.w};
+        const uint32_t upto = tab.upto[h];
+
+        // ---- the rest of the row: F and H, the row maximum, the new words ----
+        phase_b(a, rs, pc, nh, h2);
+        const uint32_t hl = __shfl_up_sync(kAll, h2[3], 1, G);
+        int32_t kk[8];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const uint32_t v = h2[p] & left[p];
+            kk[p] = (int32_t)(v * sp.k16 + (uint32_t)p);
+            kk[p + 4] = (int32_t)prmt((uint32_t)(p + 4), v, 0x7610u);
+        }
+        key = max3_i32(max3_i32(kk[0], kk[1], kk[2]), max3_i32(kk[3], kk[4], kk[5]), max(kk[6], kk[7])) + col0;
+        key = max_of_group<G>(key);
+        nh[0] = prmt(r ? hl : (uint32_t)h1 << 16, h2[3], 0x5432u);
+        // columns beyond end keep their words, column end has E = 0 (ksw.cu:371)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            H[p] = (nh[p] & ~right[p]) | (H[p] & right[p]);
+            E[p] = (ne[p] & left[p]) | (E[p] & right[p]);
+        }
+        const uint32_t nz = nonzero_mask(H, E, upto);
+        const unsigned bal = __ballot_sync(kAll, nz != 0u) & gmask;
+        fl = ffs32(bal) - 1;
+        ll = msb32(bal);
+        nzf = __shfl_sync(kAll, nz, fl & 31);
+        nzl = __shfl_sync(kAll, nz, ll & 31);
+        // to-end score: H(i, qlen - 1) is the H word of column qlen (used in its lane only); an
+        // empty row ends at beg with h1
+        {
+            const bool w2 = (J.qlen & 2) != 0;
+            const int32_t v = (int32_t)prmt(w2 ? H[2] : H[0], w2 ? H[3] : H[1], J.qsel);
+            gval = max(beg, end) == J.qlen ? (beg < end ? v : h1) : kNoGscore;
+        }
+        // the column that the band clamp cuts off in row i + 1 (ksw.cu:338) becomes zero
+        const int cc = cut - col0;
+        if (__any_sync(kAll, shr_clamp(nz, (uint32_t)cc) & 1u)) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint32_t keep = cc == p ? 0xFFFF0000u : cc == p + 4 ? 0x0000FFFFu : 0xFFFFFFFFu;
+                H[p] &= keep;
+                E[p] &= keep;
+            }
+        }
+        ++J.i;
+    }
+    busy += rows;
+    idle += (lane == 0 ? (unsigned long long)iters * kGroups : 0ull) - rows;
+}
+
+// d.order null and d.order_off null: jobs 0 .. n in the given order (or d.order's), one warp each;
+// misfit non-null (see run_groups).  Else classes 0-3 of a sorted batch (order_off: [offset,
+// count] pairs), widest first.
+template <bool kSym>
+__global__ void __launch_bounds__(32 * kBlockWarps) group16_kernel(LaunchDesc d, ScoreParams sp, int32_t* misfit,
+                                                                  int32_t* misfits) {
+    pdl_trigger();
+    __shared__ EdgeTable tab;
+    __shared__ uint2 pools[8];
+    for (int t = threadIdx.x; t < 10; t += 32 * kBlockWarps) {
+        const int h = t - 1;
+        uint32_t lw[4], rw[4];
+        for (int p = 0; p < 4; ++p) {
+            lw[p] = ~ge_word(h < 0 ? 0 : h, p);
+            rw[p] = ge_word(h + 1, p);
+        }
+        tab.left[t] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        tab.right[t] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+        tab.upto[t] = h < 0 ? 0u : (h < 8 ? (2u << h) - 1u : 0xFFu) & 0xFFu;
+    }
+    if (threadIdx.x < 8) {
+        uint32_t lo[5], hi[5];
+        score_pools(sp, lo, hi);
+        const int a = threadIdx.x < 4 ? threadIdx.x : 4;
+#pragma unroll
+        for (int t = 0; t < 5; ++t)
+            if (a == t) pools[threadIdx.x] = make_uint2(lo[t], hi[t]);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const PairConst pc = pair_const(sp);
+    unsigned long long busy = 0, idle = 0, waves = 0;
+    if (!d.order_off) {
+        const int n = d.count ? *d.count : d.n;
+        run_groups<32, kSym>(d, sp, pc, tab, pools, d.order, n, d.queue, misfit, misfits, lane, busy, idle, waves);
+    } else {
+        const int32_t* oc = d.order_off;
+        run_groups<32, kSym>(d, sp, pc, tab, pools, d.order + oc[6], oc[7], d.queue + 3, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<16, kSym>(d, sp, pc, tab, pools, d.order + oc[4], oc[5], d.queue + 2, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<8, kSym>(d, sp, pc, tab, pools, d.order + oc[2], oc[3], d.queue + 1, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<4, kSym>(d, sp, pc, tab, pools, d.order + oc[0], oc[1], d.queue, nullptr, nullptr, lane, busy, idle, waves);
+    }
+    if (d.stats) add_warp_stats(d.stats, busy, idle, waves, lane);
+    pdl_chain_end();
+}
+
+}  // namespace
+
+// The classes of a sorted group16 batch: queries up to 8 G - 1 bases in groups of G lanes, then
+// everything the groups cannot take.
+void group16_tiles(TileTable& t) {
+    const int w[] = {31, 63, 127, 255, 0x7FFFFFFF};
+    t.n = 5;
+    for (int k = 0; k < 5; ++k) {
+        t.width[k] = w[k]; t.lanes[k] = k < 4 ? 1 : 32; t.tile[k] = k < 4 ? 2 : 9;
+        t.warp_batch[k] = 0; t.refill[k] = 1;
+    }
+}
+
+int launch_group16(const LaunchDesc& d, const ScoreParams& sp, int32_t* misfit, int32_t* misfits,
+                   cudaStream_t stream) {
+    auto kern = sp.oe_del == sp.oe_ins ? group16_kernel<true> : group16_kernel<false>;
+    const int per_sm = resident_blocks(kern, 32 * kBlockWarps, 0);
+    const int need = (d.n + kBlockWarps - 1) / kBlockWarps;
+    const int full = sm_count() * (per_sm > 0 ? per_sm : 1);
+    const int blocks = need < full ? need : full;
+    if (blocks < 1) return G3X_OK;
+    kern<<<blocks, 32 * kBlockWarps, 0, stream>>>(d, sp, misfit, misfits);
+    return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
+}
+
+}  // namespace g3x

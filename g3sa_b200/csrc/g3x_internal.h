@@ -48,6 +48,7 @@ struct LaunchDesc {
     int32_t ring;          // lane-per-job kernel: 0, or the columns of its row-buffer ring
     int32_t pdl;           // class kernels: 1 = launched as a programmatic dependent of the
                            // class kernel before it on the stream (launch_class_kernel)
+    int32_t retry;         // a seed-level retry wave: few of its n jobs, a device-side count
     int64_t n_bases;       // bases the planes hold: jobs reaching past them are refused
     int64_t step_limit;    // plain (rolling) kernel: per-job step bound, 0 = the default bound
 };
@@ -242,6 +243,12 @@ int launch_lane(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream)
 int launch_lane16(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream);
 int launch_lane2(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream);
 int launch_band(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream);
+// The int16x2 group-per-job kernel (g3x_group16.cu) over the first four classes of group16_tiles,
+// or, with d.order_off null, over the jobs as they are listed; jobs it cannot take then go to
+// misfit[0 .. *misfits).  d.queue: four zeroed counters.
+void group16_tiles(TileTable& t);
+int launch_group16(const LaunchDesc& d, const ScoreParams& sp, int32_t* misfit, int32_t* misfits,
+                   cudaStream_t stream);
 size_t band_smem_per_warp(int qcap);
 size_t lane2_smem_per_warp(int qcap);
 size_t lane16_smem_per_warp(int qcap);
@@ -273,10 +280,11 @@ int extend_seeds(const SeedScratch& ws, const g3x_opt_t& opt, const ScoreParams&
                  g3x_reg_t* regs, int32_t* status, const LaunchDesc& proto, cudaStream_t st,
                  const WaveRunner* runner = nullptr);
 // What one width-class pipeline uses: the sort scratch, the classes' job-queue counters
-// (kMaxBuckets), one stream per class and the events that fork the classes from the caller's
+// (kQueueInts), one stream per class and the events that fork the classes from the caller's
 // stream and join them back (side null: the classes chain on the caller's stream as
 // programmatic dependent launches), the occupancy counters (or none).  A context has one; the seed stream keeps one per
 // chunk it runs at a time.
+constexpr int kQueueInts = 16;
 struct ClassRes {
     SchedScratch* sched;
     int32_t* queue;
@@ -295,6 +303,7 @@ struct ClassWave {
     g3x_ctx* ctx;
     bool learned;
     const ClassRes* res;
+    int32_t at_once;    // waves of this size that run side by side
 };
 int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaStream_t st);
 

@@ -170,23 +170,24 @@ int extend_seeds(const SeedScratch& ws, const g3x_opt_t& opt, const ScoreParams&
     left_jobs_kernel<<<nb, tb, 0, st>>>(seeds, n, opt, proto.n_bases, ws.ljobs, ws.order[0], ws.counters + 0,
                                         regs, status);
     auto wave = [&](g3x_job_t* jobs, g3x_ext_t* ext, int32_t* jst, int32_t* order, int32_t* count,
-                    int32_t* queue) -> int {
+                    int32_t* queue, int retry) -> int {
         LaunchDesc d = proto;
+        d.retry = retry;
         d.jobs = jobs; d.codes = codes; d.nmask = nmask; d.out = ext; d.status = jst;
         d.cells = nullptr; d.rows = nullptr; d.order = order; d.count = count; d.queue = queue; d.n = n;
         return runner ? runner->run(runner->user, d, sp, st) : launch_extend(d, sp, st);
     };
     int rc;
-    if ((rc = wave(ws.ljobs, ws.lext, ws.lstatus, ws.order[0], ws.counters + 0, ws.counters + 8))) return rc;
+    if ((rc = wave(ws.ljobs, ws.lext, ws.lstatus, ws.order[0], ws.counters + 0, ws.counters + 8, 0))) return rc;
     retry_kernel<<<nb, tb, 0, st>>>(ws.order[0], ws.counters + 0, ws.ljobs, ws.lext, ws.lstatus, 0,
                                     ws.order[1], ws.counters + 1);
-    if ((rc = wave(ws.ljobs, ws.lext, ws.lstatus, ws.order[1], ws.counters + 1, ws.counters + 9))) return rc;
+    if ((rc = wave(ws.ljobs, ws.lext, ws.lstatus, ws.order[1], ws.counters + 1, ws.counters + 9, 1))) return rc;
     left_finish_kernel<<<nb, tb, 0, st>>>(seeds, n, opt, ws.ljobs, ws.lext, ws.rjobs, ws.order[2],
                                           ws.counters + 2, regs, ws.lstatus, status);
-    if ((rc = wave(ws.rjobs, ws.rext, ws.rstatus, ws.order[2], ws.counters + 2, ws.counters + 10))) return rc;
+    if ((rc = wave(ws.rjobs, ws.rext, ws.rstatus, ws.order[2], ws.counters + 2, ws.counters + 10, 0))) return rc;
     retry_kernel<<<nb, tb, 0, st>>>(ws.order[2], ws.counters + 2, ws.rjobs, ws.rext, ws.rstatus, 1,
                                     ws.order[3], ws.counters + 3);
-    if ((rc = wave(ws.rjobs, ws.rext, ws.rstatus, ws.order[3], ws.counters + 3, ws.counters + 11))) return rc;
+    if ((rc = wave(ws.rjobs, ws.rext, ws.rstatus, ws.order[3], ws.counters + 3, ws.counters + 11, 1))) return rc;
     right_finish_kernel<<<nb, tb, 0, st>>>(seeds, n, opt, ws.rjobs, ws.rext, regs, ws.rstatus, status);
     return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
 }

@@ -68,7 +68,7 @@ int make_lanes(StreamScratch& ss) {
         ok = cudaStreamCreateWithFlags(&s.comp, cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&s.h2d, cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) == cudaSuccess &&
-             cudaMalloc(&s.queue, kMaxBuckets * sizeof(int32_t)) == cudaSuccess;
+             cudaMalloc(&s.queue, kQueueInts * sizeof(int32_t)) == cudaSuccess;
     }
     if (!ok) {
         free_stream_scratch(ss);
@@ -162,7 +162,7 @@ int extend_seeds_stream(StreamScratch& ss, const g3x_opt_t& opt, const ScorePara
         s.pending = -1;
         if (!runner) continue;
         res[l] = ClassRes{&s.sched, s.queue, nullptr, nullptr, nullptr, nullptr};
-        cw[l] = ClassWave{cw0->ctx, cw0->learned, &res[l]};
+        cw[l] = ClassWave{cw0->ctx, cw0->learned, &res[l], (int32_t)std::min<int64_t>(nchunks, kStreamLanes)};
         wr[l] = WaveRunner{runner->run, &cw[l]};
     }
     const int64_t total_code_words = (n_bases + 15) / 16, total_mask_words = (n_bases + 31) / 32;

@@ -1,0 +1,100 @@
+"""GPU parity of the int16x2 group-per-job kernel (g3x_group16.cu), which small scheduled batches
+take on a context whose width classes were not set: against the oracle, and for every kind of job
+it may not take against the row-parallel kernel (the general path).  Sizes: queries on both sides
+of every group width (31 | 32, 63 | 64, 127 | 128, 255 | 256), batches on both sides of the limit
+up to which jobs run as they are listed (1024), and one- and two-job batches."""
+import numpy as np
+import pytest
+
+import g3sa_b200 as g
+from tests import native as nat
+from tests.gpu_util import to_dev
+
+pytestmark = pytest.mark.gpu
+
+SCORES = {"bwa": {}, "uneven": dict(o_del=5, e_del=2, o_ins=7, e_ins=1), "steep": dict(a=3, b=2, o_del=1, e_del=30, o_ins=1, e_ins=40),
+          "nozdrop": dict(zdrop=0)}
+
+
+def run(u8, jobs, sc, schedule=g.SCHED_SORTED, kernel=g.KERNEL_AUTO, mq=None, mt=None, n_bases=None, rows=True):
+    import torch
+    c = g.Context(0)
+    n = len(jobs)
+    codes, nmask = g.pack_planes(u8)
+    out = torch.full((n, 6), -777, dtype=torch.int32, device="cuda")
+    status = torch.full((n,), 99, dtype=torch.int32, device="cuda")
+    cells = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    d_rows = torch.full((n,), -1, dtype=torch.int32, device="cuda") if rows else None
+    c.extend_batch(sc, to_dev(jobs), n, to_dev(codes), to_dev(nmask), out, status,
+                   int(jobs["qlen"].max()) if mq is None else mq, int(jobs["tlen"].max()) if mt is None else mt,
+                   schedule=schedule, kernel=kernel, d_cells=cells if rows else None, d_rows=d_rows, n_bases=n_bases)
+    torch.cuda.synchronize()
+    stats = c.last_stats()
+    res = [t.cpu().numpy() for t in (out, status, cells)]
+    c.close()
+    return res + [d_rows.cpu().numpy() if rows else None, stats]
+
+
+def edge_jobs(n, seed, w):
+    """Jobs of the long generator cut to query lengths around the group widths and to targets from
+    none to twice the query; reversed reads among them."""
+    wl = g.synth(4, n // 4 + 1, seed=seed, w=w, unrelated=0.0)
+    rng = np.random.default_rng(seed)
+    jobs = np.repeat(wl.jobs, 4)[:n].copy()
+    edges = [0, 1, 2, 7, 8, 9, 15, 16, 17, 30, 31, 32, 33, 62, 63, 64, 65, 126, 127, 128, 129, 200, 254, 255, 256, 257, 300]
+    jobs["qlen"] = rng.choice(edges, n)
+    jobs["tlen"] = np.minimum(jobs["tlen"], rng.choice([0, 1, 15, 16, 17, 64, 300, 480], n))
+    jobs["h0"] = rng.choice([0, 1, 5, 19, 60, 150], n)
+    jobs["w"] = rng.choice([1, 3, w], n)
+    jobs["flags"] = rng.integers(0, 4, n)
+    return wl.u8, jobs
+
+
+@pytest.mark.parametrize("score", list(SCORES))
+@pytest.mark.parametrize("n", [1, 2, 63, 1024, 1025, 6000])
+def test_edges_match_oracle(score, n):
+    sc = g.default_score(**SCORES[score])
+    u8, jobs = edge_jobs(n, 17 + n, 40)
+    ref, cells, rows = nat.oracle_extend(jobs, u8, sc)
+    out, status, gcells, grows, _ = run(u8, jobs, sc)
+    assert (status == 0).all()
+    np.testing.assert_array_equal(out, ref)
+    np.testing.assert_array_equal(gcells, cells)
+    np.testing.assert_array_equal(grows, rows)
+
+
+@pytest.mark.parametrize("kind,w,units", [(1, 100, 900), (1, 5, 20000), (2, 100, 500), (2, 100, 12000), (2, 13, 12000)])
+@pytest.mark.parametrize("score", ["bwa", "uneven"])
+def test_generated_jobs_match_oracle(kind, w, units, score):
+    sc = g.default_score(**SCORES[score])
+    wl = g.synth(kind, units, seed=units + w, w=w, unrelated=0.3)
+    ref, cells, rows = nat.oracle_extend(wl.jobs, wl.u8, sc)
+    out, status, gcells, grows, stats = run(wl.u8, wl.jobs, sc)
+    assert (status == 0).all() and stats[0] > 0
+    np.testing.assert_array_equal(out, ref)
+    np.testing.assert_array_equal(gcells, cells)
+    np.testing.assert_array_equal(grows, rows)
+    out, status, _, _, _ = run(wl.u8, wl.jobs, sc, rows=False)
+    np.testing.assert_array_equal(out, ref)
+
+
+@pytest.mark.parametrize("n", [200, 3000])
+def test_refused_and_misfit_jobs_as_on_the_general_path(n):
+    sc = g.default_score()
+    u8, jobs = edge_jobs(n, 5, 40)
+    rng = np.random.default_rng(n)
+    k = rng.permutation(n)
+    jobs["h0"][k[:20]] = 20000                        # outside int16
+    jobs["h0"][k[20:30]] = -1                         # refused
+    jobs["h0"][k[30:40]] = -50000                     # negative and taken
+    jobs["q_off"][k[40:50]] = len(u8) - 3             # past the planes
+    jobs["t_off"][k[50:60]] = 0xFFFFFFF0
+    jobs["h0"][k[60:70]] = 2000000
+    want = run(u8, jobs, sc, kernel=g.KERNEL_ROWPAR, mq=260, mt=400, n_bases=len(u8))
+    got = run(u8, jobs, sc, mq=260, mt=400, n_bases=len(u8))
+    # a job both too long and past the planes may be refused as either
+    both = (jobs["qlen"] > 260) | (jobs["tlen"] > 400)
+    np.testing.assert_array_equal(got[1][~both], want[1][~both])
+    assert ((got[1] != 0) == (want[1] != 0)).all()
+    for a, b in zip(got[:1] + got[2:4], want[:1] + want[2:4]):
+        np.testing.assert_array_equal(a, b)
