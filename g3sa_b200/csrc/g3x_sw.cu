@@ -58,6 +58,11 @@ struct SwDesc {
     int32_t xtra, maxmat;
     uint32_t tab[10];          // per target base: score bytes (lo: codes 0-3, hi: N, then 0)
     uint32_t nedel, noedel, neins, noeins;   // -e_del, -(o_del+e_del), ... as int16x2
+    // the carried F (sw_rows): its decay of segment 0 and the step to the next segment's, e_ins to
+    // add, and 1 (a run-time value keeps the step a multiply-add, beside the saturated ALU pipe);
+    // one == 0: the WIDE form, with nstep the saturating step.  carry_e: the decay per segment.
+    uint32_t dec0, step, peins, one, nstep;
+    int32_t carry_e;
     int64_t n_bases;           // bases the planes hold: jobs reaching past them are refused
 };
 
@@ -115,6 +120,21 @@ struct Rows {
     }
 };
 
+// Selectors of the segments' scores: one per register up to 16 segments, two beyond (registers
+// bound the resident warps there).
+__host__ __device__ constexpr int sel_words(int maxseg) { return maxseg > 16 ? maxseg / 2 : maxseg; }
+template <int MAXSEG, int S>
+__device__ __forceinline__ uint32_t sel_at(const uint32_t (&sel)[sel_words(MAXSEG)]) {
+    if constexpr (MAXSEG <= 16) return sel[S];
+    else return (S & 1) ? sel[S >> 1] >> 16 : sel[S >> 1];
+}
+
+// The int16x2 word of -v in both halves, at most 2^15 - 1.
+__device__ __forceinline__ uint32_t neg_pair(int64_t v) {
+    const uint32_t n = (uint32_t)-(int32_t)(v < 0x7FFF ? v : 0x7FFF) & 0xFFFFu;
+    return n | n << 16;
+}
+
 struct PassOut {
     int score, te, qe;
 };
@@ -124,39 +144,66 @@ struct PassOut {
 #define G3X_SW_CASES(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) \
     F(15) F(16) F(17) F(18) F(19) F(20) F(21) F(22) F(23) F(24) F(25) F(26) F(27) F(28) F(29) F(30) F(31)
 
+// Constants of a pass: the score steps of SwDesc as int16x2 and what a job's segment count makes of
+// the insertion extension.
+struct PassConst {
+    uint32_t last;             // decay of the carried F up to the last segment
+    uint32_t d1, d2, d4;       // decay of F over 1, 2 and 4 cells of the vector (slen segments each)
+};
+
 // The row loop of one pass over registers H, E (slot MAXSEG - slen + j = segment j).  UNI: every
 // live quad of the warp has the same slot base, so no slot needs a per-quad guard; a quad that
-// is not running computes on slots it never reads back.
-template <int MAXSEG, bool UNI, bool SYM>
+// is not running computes on slots it never reads back.  SYM: equal insertion and deletion costs,
+// so E and F share H - (o + e).  WIDE: see below.
+//
+// The lazy-F loop (ksw.cu:209-220) in closed form.  It moves F up one cell, folds it into H segment
+// by segment as it decays, E untouched, round after round, until no cell's F - e beats its
+// H - (o + e).  With o > 0 it can only stop where every F it still holds is dominated by the F
+// that the row's own pass had computed from there on (F > H - o - e fails for a cell that F itself
+// has just raised), so stopping early changes nothing and the loop's result is
+//   H(j) = max(H(j), C - j e),   C(cell) = max over the cells before it of their F at the end of
+//                                the pass, less slen e per cell in between.
+// C is a prefix over the vector's eight cells, three shuffles a row, and the row maximum and the
+// best row's position never come from a raised cell (it stays below the H it descends from).  So
+// H is stored as the pass leaves it, and the next row raises each segment as it reads it (one
+// addition and maximum) -- no loop, no ballot.  The decay -(j + 1) e of segment j (C is kept as
+// C + e) is one 32-bit addition a segment on both halves, exact while it fits 16 bits.  WIDE: gap
+// extensions above 1000 decay C by a saturating step instead; so does o = 0, where the loop stops
+// after the first segment of the first round and raises nothing else.
+template <int MAXSEG, bool UNI, bool SYM, bool WIDE>
 __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Rows& rows, int minsc, int endsc,
                                         uint32_t* sub, int& n_b, uint32_t (&H)[MAXSEG], uint32_t (&E)[MAXSEG],
-                                        const uint32_t (&sel2)[MAXSEG / 2], int base, int base_min, uint32_t* hm,
-                                        const uint32_t* tab, int lane, int& gmax, int& te) {
+                                        const uint32_t (&sel)[sel_words(MAXSEG)], const PassConst& pc, int base,
+                                        int base_min, uint32_t* hm, const uint2* tab, int lane, int& gmax, int& te) {
     const int p = lane & 3;
-    const unsigned qmask = 0xFu << (lane & ~3);
     int last_row = -2, last_v = 0;
     bool run = live;
+    uint32_t fc = 0u;             // the carried F of the row before (WIDE: C, else C + e_ins)
     for (int i = 0;; ++i) {
         run = run && i < tlen;
         if (!__any_sync(kFull, run)) break;
-        uint32_t lo = 0u, hi = 0u;
-        if (run) {
-            const uint32_t t = rows.code(d.codes, d.nmask, i);
-            lo = tab[2 * t]; hi = tab[2 * t + 1];
-        }
-        uint32_t hd = shift_up(H[MAXSEG - 1], p);
-        uint32_t f = 0u, mx = 0u;
+        uint2 pool = make_uint2(0u, 0u);
+        if (run) pool = tab[rows.code(d.codes, d.nmask, i)];
+        uint32_t hd = shift_up(__viaddmax_s16x2(fc, pc.last, H[MAXSEG - 1]), p);
+        uint32_t f = 0u, mx = 0u, dec = d.dec0;
         // the row (ksw.cu:193-208): M = H(i-1, j-1) + S, H = max(M, E, F), E' and F' from H
         switch (base_min) {
 #define G3X_SW_MAIN(S)                                                                               \
     case S:                                                                                          \
         if constexpr (S < MAXSEG) {                                                                  \
             if (UNI || S >= base) {                                                                  \
-                const uint32_t sc = prmt(lo, hi, (S & 1) ? sel2[S >> 1] >> 16 : sel2[S >> 1]);         \
+                const uint32_t sc = prmt(pool.x, pool.y, sel_at<MAXSEG, S>(sel));                    \
                 const uint32_t h = __viaddmax_s16x2(hd, sc, __vimax_s16x2_relu(E[S], f));            \
-                mx = __vimax_s16x2_relu(mx, h);                                                      \
-                hd = H[S];                                                                           \
+                if constexpr (WIDE) {                                                                \
+                    hd = __vimax_s16x2_relu(H[S], fc);                                               \
+                    fc = __viaddmax_s16x2_relu(fc, d.nstep, 0u);                                     \
+                } else {                                                                             \
+                    hd = __viaddmax_s16x2(fc, dec, H[S]);                                            \
+                    dec = dec * d.one + d.step;                                                      \
+                }                                                                                    \
                 H[S] = h;                                                                            \
+                /* two segments at a time (a slot before the job's first holds zeros) */            \
+                if constexpr (S & 1) mx = __vimax3_s16x2(mx, H[S - 1], h);                           \
                 const uint32_t td = __viaddmax_s16x2_relu(h, d.noedel, 0u);                          \
                 E[S] = __viaddmax_s16x2(E[S], d.nedel, td);                                          \
                 f = __viaddmax_s16x2(f, d.neins, SYM ? td : __viaddmax_s16x2_relu(h, d.noeins, 0u)); \
@@ -166,41 +213,12 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
 #undef G3X_SW_MAIN
             default: break;
         }
-        // lazy F (ksw.cu:209-220): at most 16 rounds of the F vector moved up one cell, then
-        // H = max(H, F) segment by segment, E untouched, until a segment where no cell's F - e
-        // beats its H - (o + e).  One ballot per segment gives every quad its stop; the warp
-        // looks for the end every other segment (a stopped quad's steps change nothing).
-        f = run ? f : 0u;
-        // A quad that stops gets F = 0, which leaves its H unchanged and keeps it stopped; a quad
-        // whose first segment is later (not UNI) waits with its F; the warp leaves when no quad
-        // goes on.
-        for (int round = 0; round < 16; ++round) {
-            f = shift_up(f, p);
-            switch (base_min) {
-#define G3X_SW_LAZY(S)                                                                               \
-    case S:                                                                                          \
-        if constexpr (S < MAXSEG) {                                                                  \
-            bool go;                                                                                 \
-            const bool at = UNI || S >= base;                                                        \
-            if (at) {                                                                                \
-                const uint32_t h = __vimax_s16x2_relu(H[S], f);                                      \
-                H[S] = h;                                                                            \
-                f = __viaddmax_s16x2_relu(f, d.neins, 0u);                                           \
-                const uint32_t hp = __viaddmax_s16x2_relu(h, d.noeins, 0u);                          \
-                go = __vimax_s16x2_relu(f, hp) != hp;                                                \
-            } else {                                                                                 \
-                go = f != 0u;                                                                        \
-            }                                                                                        \
-            const unsigned bal = __ballot_sync(kFull, go);                                           \
-            if (at && !(bal & qmask)) f = 0u;                                                        \
-            if ((S & 1) && !bal) goto lazy_done;                                                     \
-        }
-                G3X_SW_CASES(G3X_SW_LAZY)
-#undef G3X_SW_LAZY
-                default: break;
-            }
-        }
-    lazy_done:
+        // the F carried into each cell (a lane a shuffle leaves alone meets its own, decayed)
+        f = shift_up(f, p);
+        f = __viaddmax_s16x2(shift_up(f, p), pc.d1, f);
+        f = __viaddmax_s16x2(__shfl_up_sync(kFull, f, 1, 4), pc.d2, f);
+        f = __viaddmax_s16x2(__shfl_up_sync(kFull, f, 2, 4), pc.d4, f);
+        fc = WIDE ? f : __viaddmax_s16x2(f, d.peins, 0u);
         uint32_t m2 = __vimax_s16x2_relu(mx, __shfl_xor_sync(kFull, mx, 1));
         m2 = __vimax_s16x2_relu(m2, __shfl_xor_sync(kFull, m2, 2));
         const int im = max((int)(int16_t)(m2 & 0xFFFFu), (int)(int16_t)(m2 >> 16));
@@ -238,13 +256,13 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
 template <int MAXSEG, typename QCode>
 __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen, int tlen, QCode qcode, Rows rows,
                                            int minsc, int endsc, uint32_t* sub, int* nb, uint32_t* hm,
-                                           const uint32_t* tab, int lane) {
+                                           const uint2* tab, int lane) {
     const int p = lane & 3;
     const int slen = live ? (qlen + 7) >> 3 : 0;
     const int base = MAXSEG - slen;
     const int base_min = (int)__reduce_min_sync(kFull, (unsigned)base);
     const bool uni = __all_sync(kFull, !live || base == base_min);
-    uint32_t H[MAXSEG], E[MAXSEG], sel2[MAXSEG / 2];
+    uint32_t H[MAXSEG], E[MAXSEG], sel[sel_words(MAXSEG)];
 #pragma unroll
     for (int s = 0; s < MAXSEG; s += 2) {
         uint32_t v = 0;
@@ -259,19 +277,32 @@ __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen,
             }
             v |= sel_of(c0, c1) << (16 * u);
         }
-        sel2[s >> 1] = v;
+        if constexpr (MAXSEG <= 16) {
+            sel[s] = v & 0xFFFFu;
+            sel[s + 1] = v >> 16;
+        } else {
+            sel[s >> 1] = v;
+        }
         H[s] = H[s + 1] = 0u;
         E[s] = E[s + 1] = 0u;
     }
     int gmax = 0, te = -1, n_b = 0;
-    // SYM: equal insertion and deletion costs, so E and F share H - (o + e)
-    if (d.noedel == d.noeins) {
-        if (uni) sw_rows<MAXSEG, true, true>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel2, base, base_min, hm, tab, lane, gmax, te);
-        else sw_rows<MAXSEG, false, true>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel2, base, base_min, hm, tab, lane, gmax, te);
+    const int64_t seg = (int64_t)slen * d.carry_e;
+    const bool wide = d.one == 0u;
+    const PassConst pc{neg_pair(wide ? seg - d.carry_e : seg), neg_pair(seg), neg_pair(2 * seg), neg_pair(4 * seg)};
+#define G3X_SW_ROWS(UNI, SYM, WIDE)                                                                              \
+    sw_rows<MAXSEG, UNI, SYM, WIDE>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel, pc, base, base_min, hm, \
+                                    tab, lane, gmax, te)
+    if (wide) {
+        G3X_SW_ROWS(false, false, true);
+    } else if (d.noedel == d.noeins) {
+        if (uni) G3X_SW_ROWS(true, true, false);
+        else G3X_SW_ROWS(false, true, false);
     } else {
-        if (uni) sw_rows<MAXSEG, true, false>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel2, base, base_min, hm, tab, lane, gmax, te);
-        else sw_rows<MAXSEG, false, false>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel2, base, base_min, hm, tab, lane, gmax, te);
+        if (uni) G3X_SW_ROWS(true, false, false);
+        else G3X_SW_ROWS(false, false, false);
     }
+#undef G3X_SW_ROWS
     __syncwarp();
     // end on the query: the smallest position holding the best row's largest cell, cells read
     // as uint16 (ksw.cu:244-248); with no best row the cells are all 0 and it is position 0
@@ -300,13 +331,13 @@ __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen,
 }
 
 template <int MAXSEG>
-__global__ void __launch_bounds__(128) sw_kernel(SwDesc d) {
+__global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) sw_kernel(SwDesc d) {
     constexpr int QMAX = 8 * MAXSEG;
     __shared__ __align__(16) uint8_t qcodes[kWarps][kQuads][QMAX];
     __shared__ uint32_t snap[kWarps][MAXSEG * 32];
-    __shared__ uint32_t tab[10];
+    __shared__ uint2 tab[5];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane >> 2, p = lane & 3;
-    if (threadIdx.x < 10) tab[threadIdx.x] = d.tab[threadIdx.x];
+    if (threadIdx.x < 5) tab[threadIdx.x] = make_uint2(d.tab[2 * threadIdx.x], d.tab[2 * threadIdx.x + 1]);
     __syncthreads();
     uint8_t* qc = qcodes[warp][quad];
     uint32_t* hm = snap[warp];
@@ -520,6 +551,13 @@ extern "C" int g3x_ksw_align2_batch(g3x_ctx* ctx, const g3x_score_t* score, cons
     }
     d.nedel = pack16(-sp.e_del); d.noedel = pack16(-sp.oe_del);
     d.neins = pack16(-sp.e_ins); d.noeins = pack16(-sp.oe_ins);
+    d.one = sp.o_ins > 0 && sp.e_ins <= 1000 ? 1u : 0u;
+    d.carry_e = sp.o_ins > 0 ? sp.e_ins : 0x7FFF;
+    // two's complement of both halves at once: -k in each is 2^16 - k (2^16 + 1)
+    d.step = 0u - (uint32_t)sp.e_ins * 0x10001u;
+    d.dec0 = 0x10000u + d.step;
+    d.peins = pack16(sp.e_ins);
+    d.nstep = pack16(-d.carry_e);
     int sms = 0;
     sms = sm_count();
     if ((rc = launch_class<32>(d, range, queue, sms, st))) return rc;

@@ -131,3 +131,20 @@ def test_gpu_sw_edge_of_int16_domain():
         assert (st == 0).all()
         assert np.array_equal(got, want)
         assert int(got["score"][0]) == 127 * 256
+
+
+@pytest.mark.parametrize("o,e", [(0, 1), (0, 7), (1, 1), (6, 999), (6, 1000), (6, 1001), (3, 30000), (32766, 1)])
+@pytest.mark.parametrize("max_q", [64, 128, 256])
+def test_gpu_sw_carried_f_at_the_edges_of_its_forms(o, e, max_q):
+    """The closed form of the lazy-F loop: insertion openings of 0 (the loop stops after one segment)
+    and extensions on both sides of the limit of its 16-bit decay (1000), equal and unequal to
+    the deletion's, on windows with long insertions, in every class of segments."""
+    cj, u8 = nat.sw_jobs(1500, 0xF0 + max_q + o + e, flank=max_q // 3, max_q=max_q)
+    for sc in (g.default_score(a=5, b=3, o_del=o, e_del=e, o_ins=o, e_ins=e),
+               g.default_score(a=20, b=1, o_del=4, e_del=2, o_ins=o, e_ins=e)):
+        for x in (0, g.KSW_XSTART | g.KSW_XSUBO | 30):
+            want, _ = nat.oracle_sw(cj, u8, sc, x)
+            got, st = run_sw(gpu_jobs(cj), u8, sc, x)
+            assert (st == 0).all()
+            bad = np.nonzero(got != want)[0]
+            assert bad.size == 0, f"xtra {x:#x}: jobs {bad[:5]}: {got[bad[:2]]} vs {want[bad[:2]]}"
