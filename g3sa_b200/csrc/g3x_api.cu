@@ -38,16 +38,12 @@ GlobalScratch& ctx_global(g3x_ctx* ctx) { return ctx->global; }
 SwScratch& ctx_sw(g3x_ctx* ctx) { return ctx->sw; }
 
 
-// The jobs in decreasing order of row count, then of widest row (the counting sort of the
-// scheduled batches with one class), so that the jobs a warp takes together are alike.
-int cost_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, const ScoreParams& sp, cudaStream_t st,
-               const int32_t** order) {
+int pair_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, int classes, cudaStream_t st, const int32_t** order,
+               const int32_t** range) {
     int rc = alloc_sched(ctx->sched, n);
-    if (rc) return rc;
-    TileTable t;
-    t.n = 1; t.width[0] = 0x7FFFFFFF; t.lanes[0] = 32; t.tile[0] = 9; t.warp_batch[0] = 0; t.refill[0] = 1;
-    if ((rc = schedule_jobs(ctx->sched, jobs, n, sp, nullptr, t, st))) return rc;
+    if (rc || (rc = sort_pairs(ctx->sched, jobs, n, classes, st))) return rc;
     *order = ctx->sched.order;
+    *range = ctx->sched.bucket_oc;
     return G3X_OK;
 }
 

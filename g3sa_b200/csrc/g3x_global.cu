@@ -1,6 +1,9 @@
 // g3x_global.cu -- banded global alignment with backtrack (ksw_global2, bwa/src/ksw.cu:706-809)
 // for batches of alignments on the GPU.
 //
+// Two kernels.  Jobs whose band fits a group of lanes and whose scores fit int16 run in
+// g3x_global16.cu; this file holds the call and the kernel for the others.
+//
 // One job per lane.  The jobs are first ordered by decreasing row count and row width (the
 // scheduler's counting sort); a warp takes 32 consecutive ones and runs their target rows
 // together (row i of every job in the same step); in a row each lane walks its own band
@@ -19,42 +22,13 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "g3x_core.h"
+#include "g3x_global.cuh"
 #include "g3x_internal.h"
 #include "g3x_stage.cuh"
 
 namespace g3x {
 
 namespace {
-
-constexpr int32_t kNegInf = -0x40000000;
-
-struct GlobalDesc {
-    const g3x_job_t* jobs;
-    const uint32_t* codes;
-    const uint32_t* nmask;
-    int32_t* score;
-    uint32_t* cigar;
-    int32_t* n_cigar;
-    int32_t* status;
-    uint8_t* z;            // direction bytes: per warp slot zwarp bytes
-    int64_t zwarp;
-    int32_t* queue;
-    const int32_t* order;  // queue slot -> job, jobs alike in row count and width together
-    int32_t* nm;           // optional: NM per job
-    char* md;              // optional: MD string per job, md_stride bytes each
-    int32_t n, qmax, tmax, wmax, ncol, ring, stride, md_stride;
-    int64_t n_bases;       // bases the planes hold: jobs reaching past them are refused
-};
-
-// Appends the decimal digits of v (>= 0) to buf[l ...] while they fit below cap.
-__device__ __forceinline__ bool put_uint(char* buf, int& l, int cap, int v) {
-    char tmp[12];
-    int k = 0;
-    do { tmp[k++] = (char)('0' + v % 10); v /= 10; } while (v);
-    if (l + k >= cap) return false;
-    while (k) buf[l++] = tmp[--k];
-    return true;
-}
 
 __device__ __forceinline__ int32_t sbyte0(uint32_t x) { return (int32_t)(int8_t)(x & 0xFFu); }
 
@@ -103,17 +77,19 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
     score_pools(sp, lo, hi);
     const int32_t oe_del = sp.o_del + sp.e_del, oe_ins = sp.o_ins + sp.e_ins;
     const int R = d.ring;
+    const int n_jobs = d.range[1];
+    const int32_t* order = d.order + d.range[0];
 
     for (;;) {
         int first = 0;
         if (lane == 0) first = atomicAdd(d.queue, 32);
         first = __shfl_sync(0xFFFFFFFFu, first, 0);
-        if (first >= d.n) break;
-        const int job = first + lane < d.n ? d.order[first + lane] : d.n;
+        if (first >= n_jobs) break;
+        const int job = first + lane < n_jobs ? order[first + lane] : -1;
         int32_t qlen = 0, tlen = 0, w = 0;
         uint32_t t_off = 0, flags = 0;
         bool trev = false, live = false;
-        if (job < d.n) {
+        if (job >= 0) {
             const g3x_job_t jb = d.jobs[job];
             qlen = jb.qlen; tlen = jb.tlen; w = jb.w; flags = jb.flags;
             t_off = jb.t_off; trev = (jb.flags & G3X_JOB_TREV) != 0;
@@ -217,13 +193,9 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
             d.n_cigar[job] = full || bad ? 0 : n;
             int32_t stj = full ? G3X_ERR_TOO_LONG : bad ? G3X_ERR_INTERNAL : G3X_OK;
             if (d.nm && stj == G3X_OK) {
-                // NM and MD along the CIGAR (aux.cu:2831-2860): the query from its codes in shared
-                // memory, the target from the planes 16 codes at a time
-                const char* alpha = (flags & 4u) ? "TGCAN" : "ACGTN";
-                char* md = d.md + (int64_t)job * d.md_stride;
-                int x = 0, y = 0, u = 0, n_mm = 0, n_gap = 0, l = 0, cy = -1;
+                // the query from its codes in shared memory, the target from the planes 16 codes at a time
+                int cy = -1;
                 uint32_t ty = 0, tyn = 0;
-                bool ok = true;
                 auto qcode = [&](int p) -> uint32_t {
                     const uint32_t nib = (qn[(p >> 3) * 32 + lane] >> ((p & 7) << 2)) & 0xFu;
                     return (nib & 4u) ? 4u : nib;
@@ -232,36 +204,7 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
                     if ((p >> 4) != cy) { cy = p >> 4; load16(d.codes, d.nmask, t_off, tlen, cy, trev, ty, tyn); }
                     return ((tyn >> (p & 15)) & 1u) ? 4u : (ty >> ((p & 15) << 1)) & 3u;
                 };
-                for (int k = 0; k < n && ok; ++k) {
-                    const int op = (int)(cg[k] & 0xFu), len = (int)(cg[k] >> 4);
-                    if (op == 0) {
-                        for (int i = 0; i < len && ok; ++i) {
-                            const uint32_t tc = tcode(y + i);
-                            if (qcode(x + i) != tc) {
-                                ok = put_uint(md, l, d.md_stride - 1, u);
-                                if (ok && l + 1 < d.md_stride) md[l++] = alpha[tc]; else ok = false;
-                                ++n_mm; u = 0;
-                            } else ++u;
-                        }
-                        x += len; y += len;
-                    } else if (op == 2) {
-                        if (k > 0 && k < n - 1) {
-                            ok = put_uint(md, l, d.md_stride - 1, u);
-                            if (ok && l + 1 < d.md_stride) md[l++] = '^'; else ok = false;
-                            for (int i = 0; i < len && ok; ++i) {
-                                if (l + 1 < d.md_stride) md[l++] = alpha[tcode(y + i)]; else ok = false;
-                            }
-                            u = 0; n_gap += len;
-                        }
-                        y += len;
-                    } else if (op == 1) {
-                        x += len; n_gap += len;
-                    }
-                }
-                ok = ok && put_uint(md, l, d.md_stride - 1, u);
-                md[ok ? l : 0] = 0;
-                d.nm[job] = ok ? n_mm + n_gap : 0;
-                if (!ok) stj = G3X_ERR_TOO_LONG;
+                if (!write_nm_md(d, job, flags, cg, n, qcode, tcode)) stj = G3X_ERR_TOO_LONG;
             } else if (d.nm) {
                 d.nm[job] = 0;
                 d.md[(int64_t)job * d.md_stride] = 0;
@@ -271,6 +214,10 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
         __syncwarp();
     }
 }
+
+// Up to here the group kernel takes the jobs as they come, a warp each; beyond, sorted by band
+// width, up to sixteen a warp.
+constexpr int kDirectPairs = 1024;
 
 }  // namespace
 
@@ -314,31 +261,57 @@ extern "C" int g3x_ksw_global2_batch(g3x_ctx* ctx, const g3x_score_t* score, con
     size_t max_smem = 0;
     if (allow_max_smem(kern, &max_smem) != cudaSuccess) return G3X_ERR_CUDA;
     if (warp_smem > max_smem) return G3X_ERR_TOO_LONG;
-    const int wpb = 2 * warp_smem <= max_smem ? 2 : 1;
-    int sms = 0, per_sm = 0;
-    sms = sm_count();
-    per_sm = resident_blocks(kern, 32 * wpb, wpb * warp_smem);
-    int blocks = sms * std::max(per_sm, 1);
-    // direction bytes: tmax rows x ncol columns x 32 lanes per resident warp, at most 8 GiB
-    d.zwarp = (int64_t)d.tmax * d.ncol * 32;
+    // The group kernel takes the jobs that fit it; the lane kernel is launched when there may be
+    // others: values beyond int16, or bands beyond the widest group (a band is cut to the longer
+    // sequence).
+    const bool groups = c16, lanes = !c16 || std::min(max_w, std::max(d.qmax, d.tmax)) > kGlobalGroupMaxW;
     const int64_t cap = (int64_t)8 << 30;
-    while (blocks > 1 && (int64_t)blocks * wpb * d.zwarp > cap) blocks = blocks / 2;
-    const int64_t need = (int64_t)blocks * wpb * d.zwarp;
+    int wpb = 0, blocks = 0, gblocks = 0;
+    int64_t need = 0;
+    const int64_t zlane = (int64_t)d.tmax * d.ncol * 32, zgroup = global16_warp_bytes(d.tmax);
+    // scratch: the resident warps' directions, at most 8 GiB; the two kernels run one after the
+    // other and share it
+    if (lanes) {
+        wpb = 2 * warp_smem <= max_smem ? 2 : 1;
+        const int per_sm = resident_blocks(kern, 32 * wpb, wpb * warp_smem);
+        blocks = sm_count() * std::max(per_sm, 1);
+        while (blocks > 1 && (int64_t)blocks * wpb * zlane > cap) blocks = blocks / 2;
+        need = (int64_t)blocks * wpb * zlane;
+    }
+    const bool direct = groups && !lanes && n <= kDirectPairs;
+    if (groups) {
+        gblocks = std::min(global16_blocks(), (n + kGlobal16Warps - 1) / kGlobal16Warps);
+        while (gblocks > 1 && (int64_t)gblocks * kGlobal16Warps * zgroup > cap) gblocks = gblocks / 2;
+        need = std::max(need, (int64_t)gblocks * kGlobal16Warps * zgroup);
+    }
     GlobalScratch& gs = ctx_global(ctx);
     if (gs.bytes < need || !gs.queue) {
         cudaFree(gs.z); cudaFree(gs.queue);
         gs.z = nullptr; gs.queue = nullptr; gs.bytes = 0;
-        if (cudaMalloc(&gs.z, (size_t)need) != cudaSuccess || cudaMalloc(&gs.queue, sizeof(int32_t)) != cudaSuccess) {
+        if (cudaMalloc(&gs.z, (size_t)need) != cudaSuccess ||
+            cudaMalloc(&gs.queue, (kGlobalGroupClasses + 1) * sizeof(int32_t)) != cudaSuccess) {
             cudaFree(gs.z); gs.z = nullptr; cudaGetLastError();
             return G3X_ERR_NOMEM;
         }
         gs.bytes = need;
     }
     d.z = gs.z;
-    d.queue = gs.queue;
     const cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = cost_order(ctx, d_jobs, n, sp, st, &d.order))) return rc;
-    if (cudaMemsetAsync(gs.queue, 0, sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
-    kern<<<blocks, 32 * wpb, wpb * warp_smem, st>>>(d, sp);
+    d.range = nullptr;
+    d.order = nullptr;
+    if (!direct && (rc = pair_order(ctx, d_jobs, n, groups ? kGlobalGroupClasses : 0, st, &d.order, &d.range))) return rc;
+    if (cudaMemsetAsync(gs.queue, 0, (kGlobalGroupClasses + 1) * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
+    if (groups) {
+        GlobalDesc g = d;
+        g.zwarp = zgroup;
+        g.queue = gs.queue;
+        if ((rc = launch_global16(g, sp, gblocks, st))) return rc;
+    }
+    if (lanes) {
+        d.zwarp = zlane;
+        d.queue = gs.queue + kGlobalGroupClasses;
+        d.range += 2 * (groups ? kGlobalGroupClasses : 0);
+        kern<<<blocks, 32 * wpb, wpb * warp_smem, st>>>(d, sp);
+    }
     return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
 }

@@ -24,6 +24,7 @@
 // beyond a few thousand jobs.
 #include <cuda_runtime.h>
 #include "g3x_core.h"
+#include "g3x_group.cuh"
 #include "g3x_internal.h"
 #include "g3x_lane16.cuh"
 #include "g3x_stage.cuh"
@@ -34,7 +35,6 @@ namespace {
 
 using namespace l16;
 
-constexpr unsigned kAll = 0xFFFFFFFFu;
 constexpr int kBlockWarps = 2;
 
 // Masks by h = clamp(end - first column of the block, -1, 8), entry h + 1: the pair words of
@@ -44,54 +44,10 @@ struct EdgeTable {
     uint32_t upto[10];
 };
 
-// A decay of `steps` lanes for values held in the high half of a word; values stay below 2^15,
-// so a decay of 2^15 - 1 already leaves nothing.
-__device__ __forceinline__ int32_t decay_hi(int32_t e_ins, int steps) {
-    const int32_t v = 8 * steps * e_ins;
-    return -((v < 0x7FFF ? v : 0x7FFF) << 16);
-}
-
 // No row yet: below every row's key but those of rows without a positive cell (columns stay below
 // 256).
 constexpr int32_t kNoRow = 0xFFFF;
 constexpr int32_t kNoGscore = -2;   // no to-end score in a row: below gscore's start
-
-// Largest of the group's values, in every lane of it.
-template <int G>
-__device__ __forceinline__ int32_t max_of_group(int32_t v) {
-    if constexpr (G == 32) {
-        return __reduce_max_sync(kAll, v);
-    } else {
-#pragma unroll
-        for (int o = G / 2; o >= 1; o >>= 1) v = max(v, __shfl_xor_sync(kAll, v, o));
-        return v;
-    }
-}
-
-// Exclusive prefix over the lanes of a group of the F leaving each block (high halves of x): F
-// entering the lane's block, where a value loses 8 e_ins per lane it passes.  A lane that a
-// shuffle leaves alone meets its own value, less the decay.  For G = 32, where a row's latency
-// counts, three lanes per step (four dependent shuffles instead of six).
-template <int G>
-__device__ __forceinline__ int32_t f_entering(int32_t x, int r, int32_t e_ins) {
-    const int32_t y = __shfl_up_sync(kAll, x, 1, G);
-    int32_t f = r ? y : 0;
-    if constexpr (G < 32) {
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) f = __viaddmax_s32(__shfl_up_sync(kAll, f, o, G), decay_hi(e_ins, o), f);
-    } else {
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 2) {
-            const int32_t a = __shfl_up_sync(kAll, f, o), b = __shfl_up_sync(kAll, f, 2 * o);
-            const int32_t c = __shfl_up_sync(kAll, f, 3 * o);
-            f = __viaddmax_s32(a, decay_hi(e_ins, o), f);
-            f = __viaddmax_s32(b, decay_hi(e_ins, 2 * o), f);
-            f = __viaddmax_s32(c, decay_hi(e_ins, 3 * o), f);
-        }
-        f = __viaddmax_s32(__shfl_up_sync(kAll, f, 16), decay_hi(e_ins, 16), f);
-    }
-    return f;
-}
 
 // v >> n for any n as an unsigned shift amount: 0 from 32 on.
 __device__ __forceinline__ uint32_t shr_clamp(uint32_t v, uint32_t n) {

@@ -110,6 +110,23 @@ __global__ void scatter_kernel(const int32_t* __restrict__ bin, int n, int32_t* 
     order[at] = job_at(k, subset);
 }
 
+// Global-alignment jobs: the band class, then rows (four bins per doubling) and the widest row.
+__global__ void pair_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int classes, int32_t* __restrict__ bin,
+                                int32_t* __restrict__ hist) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const g3x_job_t jb = jobs[k];
+    const int w = min(max(jb.w, 0), (int)max(jb.qlen, jb.tlen));
+    int c = 0;
+    while (c < classes && 2 * w + 1 > 16 << c) ++c;
+    int rb = (int)((16.0f - log2f(1.0f + (float)jb.tlen)) * (kSchedRowBins / 16.0f));
+    rb = min(max(rb, 0), kSchedRowBins - 1);
+    const int wb = kSchedWidthBins - 1 - min((min((int)jb.qlen, 2 * w + 1) + 7) >> 3, kSchedWidthBins - 1);
+    const int bn = c * kLevels + rb * kSchedWidthBins + wb;
+    bin[k] = bn;
+    sched_count(hist, bn);
+}
+
 __global__ void max_w_kernel(const g3x_job_t* __restrict__ jobs, int n, ScoreParams sp, int32_t* out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int32_t w = 0;
@@ -131,6 +148,16 @@ int batch_max_w(const g3x_job_t* jobs, int n, const ScoreParams& sp, int32_t* d_
         cudaStreamSynchronize(st) != cudaSuccess)
         return G3X_ERR_CUDA;
     return G3X_OK;
+}
+
+int sort_pairs(SchedScratch& s, const g3x_job_t* jobs, int n, int classes, cudaStream_t st) {
+    const int nbins = (classes + 1) * kLevels;
+    if (cudaMemsetAsync(s.hist, 0, nbins * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
+    const int tb = 256, nb = (n + tb - 1) / tb;
+    pair_bin_kernel<<<nb, tb, 0, st>>>(jobs, n, classes, s.bin, s.hist);
+    scan_kernel<<<1, 1024, 0, st>>>(s.hist, nbins, s.cursor, s.bucket_oc, classes + 1);
+    scatter_kernel<<<nb, tb, 0, st>>>(s.bin, n, s.cursor, s.order, nullptr, nullptr);
+    return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
 }
 
 int schedule_jobs(SchedScratch& s, const g3x_job_t* jobs, int n, const ScoreParams& sp,

@@ -145,3 +145,48 @@ def test_gpu_global_both_ring_forms(long_len):
     assert np.array_equal(n1, n2)
     assert all(np.array_equal(c1[k, :n1[k]], c2[k, :n2[k]]) for k in range(len(cj)))
     assert out_of_band.any() and (s1[out_of_band] < -(1 << 29)).any()
+
+
+def pairs_at_edges(n, seed, ws, lens):
+    """Pairs cut to given lengths: targets are edited copies, shortened, lengthened or absent."""
+    rng = np.random.default_rng(seed)
+    cj, u8 = nat.global_jobs(n, seed, max_len=max(lens) + 1, ws=ws)
+    cj["qlen"] = np.minimum(cj["qlen"], rng.choice(lens, n))
+    cut = rng.random(n)
+    cj["tlen"] = np.where(cut < 0.1, 0, np.where(cut < 0.5, cj["tlen"], np.minimum(cj["tlen"], rng.choice(lens, n))))
+    return cj, u8
+
+
+@pytest.mark.parametrize("n", [1, 3, 1024, 1025, 5000])
+@pytest.mark.parametrize("score", [{}, dict(o_del=5, e_del=2, o_ins=7, e_ins=1), dict(a=6, b=9, o_del=0, e_del=5, o_ins=1, e_ins=6)])
+def test_gpu_global_group_widths(n, score):
+    """Bands on both sides of every group width (2w + 1 columns in 16, 32, 64, 128, 256; a band is
+    cut to the longer sequence) and beyond the widest, up to and beyond the batch size that runs
+    unsorted: scores, CIGARs, NM and MD equal the oracle's."""
+    import torch
+    sc = g.default_score(**score)
+    for ws in ((0, 1, 3, 4, 7, 8, 15, 16, 31, 32, 63, 64, 126, 127), (2, 7, 100, 127, 128, 200, 500)):
+        cj, u8 = pairs_at_edges(n, 31 + n, ws, (0, 1, 2, 7, 8, 9, 16, 33, 64, 127, 128, 200, 255))
+        jobs = gpu_jobs(cj)
+        stride = int((cj["qlen"] + cj["tlen"]).max()) + 2
+        md_stride = 4 * stride + 16
+        s1, c1, n1, _ = nat.oracle_global(cj, u8, sc, stride)
+        nm1, md1 = nat.oracle_nm_md(cj, u8, c1, n1, md_stride)
+        codes, nmask = g.pack_planes(u8)
+        out = [torch.full((n * k,), 77, dtype=torch.int32, device="cuda") for k in (1, stride, 1, 1, 1)]
+        d_md = torch.zeros(n * md_stride, dtype=torch.uint8, device="cuda")
+        ctx().global_batch(sc, to_dev(jobs), n, to_dev(codes), to_dev(nmask), int(cj["qlen"].max()),
+                           int(cj["tlen"].max()), int(cj["w"].max()), out[0], out[1], stride, out[2], out[3],
+                           d_nm=out[4], d_md=d_md, md_stride=md_stride)
+        torch.cuda.synchronize()
+        s2, c2, n2, st, nm2 = [t.cpu().numpy() for t in out]
+        assert (st == 0).all(), np.unique(st)
+        np.testing.assert_array_equal(s2, s1)
+        np.testing.assert_array_equal(n2, n1)
+        c2 = c2.view(np.uint32).reshape(n, stride)
+        for k in range(n):
+            assert np.array_equal(c1[k, :n1[k]], c2[k, :n2[k]]), (k, cj[k])
+            assert (c2[k, n2[k]:] == 77).all()                  # slots beyond the CIGAR stay
+        np.testing.assert_array_equal(nm2, nm1)
+        md = d_md.cpu().numpy().reshape(n, md_stride)
+        assert [bytes(md[k]).split(b"\0")[0].decode() for k in range(n)] == md1
