@@ -189,6 +189,28 @@ static ClassRes ctx_res(g3x_ctx* ctx) {
                     ctx->d_stats};
 }
 
+// The jobs of an unbounded last class (d: their order and count, on the row-parallel kernel's
+// settings).  Queries beyond the lane classes run in the band kernel where a window holds their
+// band: 1,500 segments of 500-5,000 bases at w = 500 take 32.8 ms row-parallel, which sweeps the row in
+// shared memory tile by tile, and 7.5 ms with the band's row in registers; 20,000 at w = 100 162 and
+// 21.  Shorter ones are here only for their scores, a few jobs not worth three launches.  queue:
+// four zeroed counters.
+static int launch_last(const LaunchDesc& d, const ScoreParams& sp, int32_t* queue, cudaStream_t st) {
+    LaunchDesc r = d;
+    r.queue = queue;
+    r.split = d.qmax > 256;
+    int rc = launch_rowpar(r, sp, st);
+    if (!r.split) return rc;
+    r.kernel = kKernelBand;
+    r.pdl = 1;
+    for (int win = 1024; win >= 256 && rc == G3X_OK; win /= 2) {
+        r.tile = win;
+        r.queue = ++queue;
+        rc = launch_band(r, sp, st);
+    }
+    return rc;
+}
+
 // Runs the persistent kernels over every width class of an ordered batch: one launch per class,
 // chained on `st` (or forked onto side streams from `st` and joined back).
 static int launch_classes(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams& sp, cudaStream_t st,
@@ -245,7 +267,9 @@ static int launch_classes(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParam
             rc = launch_band(d, sp, cs);
         } else {
             while (d.lanes < 32 && (32 / d.lanes) * group_smem_bytes(d.qmax, d.tmax) > 227 * 1024) d.lanes *= 2;
-            rc = launch_rowpar(d, sp, cs);
+            rc = k == tt.n - 1 && !ctx->tiles_set && !tt_override
+                     ? launch_last(d, sp, res.queue + kMaxBuckets, cs)
+                     : launch_rowpar(d, sp, cs);
         }
         if (rc == G3X_OK && timed) {
             if (cudaEventRecord(ctx->cls1[k], cs) != cudaSuccess) rc = G3X_ERR_CUDA;
@@ -305,12 +329,11 @@ static int run_grouped(const LaunchDesc& base, const ScoreParams& sp, SchedScrat
     }
     if (rc) return rc;
     rest.order = s.order;
-    rest.queue = queue + 8;
     rest.kernel = kKernelRowpar;
     rest.lanes = 32; rest.tile = 9; rest.warp_batch = 0; rest.refill = 1;
     rest.persistent = 1; rest.warps_per_block = 4;
     rest.pdl = !direct;
-    return launch_rowpar(rest, sp, st);
+    return launch_last(rest, sp, queue + 4, st);
 }
 
 // Schedules and runs a persistent batch: cost per job (length, or the model's prediction),
@@ -331,7 +354,7 @@ static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams
                                      ctx->model.params, sp, ctx->tiles, st)
              : schedule_jobs(ctx->sched, base.jobs, base.n, sp, nullptr, ctx->tiles, st);
     if (rc) return rc;
-    if (cudaMemsetAsync(ctx->d_queue, 0, kMaxBuckets * sizeof(int32_t), st) != cudaSuccess ||
+    if (cudaMemsetAsync(ctx->d_queue, 0, kQueueInts * sizeof(int32_t), st) != cudaSuccess ||
         cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), st) != cudaSuccess)
         return G3X_ERR_CUDA;
     return launch_classes(ctx, base, sp, st);
@@ -351,7 +374,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
                                          ctx->tiles, st, d.order, d.count)
                  : schedule_jobs(sched, d.jobs, d.n, sp, nullptr, ctx->tiles, st, d.order, d.count);
     if (rc) return rc;
-    if (cudaMemsetAsync(res.queue, 0, kMaxBuckets * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
+    if (cudaMemsetAsync(res.queue, 0, kQueueInts * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
     LaunchDesc base = d;
     base.order = nullptr; base.count = nullptr; base.order_off = nullptr; base.queue = nullptr;
     return launch_classes(ctx, base, sp, st, -1, nullptr, w->res);

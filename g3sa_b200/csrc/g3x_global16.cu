@@ -42,20 +42,6 @@ using namespace l16;
 
 constexpr int32_t kBias = 0x4000;
 
-// Codes of query positions c .. c + 7 as nibbles (0 outside [0, qlen)).
-__device__ __forceinline__ uint32_t codes8(const GlobalDesc& d, uint32_t off, int qlen, bool rev, int c) {
-    const int ch = c >> 4, sh = (c & 15) << 2;
-    uint64_t v[2] = {0, 0};
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-        if (ch + u >= 0 && (ch + u) << 4 < qlen && (u == 0 || sh > 32)) {
-            uint32_t x, nb;
-            load16(d.codes, d.nmask, off, qlen, ch + u, rev, x, nb);
-            v[u] = nibbles16(x, nb);
-        }
-    return (uint32_t)(v[0] >> sh) | (sh > 32 ? (uint32_t)(v[1] << (64 - sh)) : 0u);
-}
-
 // One 16-bit half of the block words, offset t of the block.
 __device__ __forceinline__ int32_t half_of(const uint32_t (&w)[4], int t) {
     const uint32_t lo = (t & 1) ? w[1] : w[0], hi = (t & 1) ? w[3] : w[2];
@@ -127,7 +113,7 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
         }
         // query codes of the block's columns and of the next eight; ext: lane r holds the eight
         // codes that enter the window at its right end in rows 8 (e0 + r) ..
-        uint32_t qlo = rows ? codes8(d, q_off, qlen, qrev, 8 * r - w) : 0u, qhi = 0u, ext = 0u, tw = 0u, t8 = 0u;
+        uint32_t qlo = rows ? codes8(d.codes, d.nmask, q_off, qlen, qrev, 8 * r - w) : 0u, qhi = 0u, ext = 0u, tw = 0u, t8 = 0u;
         uint32_t* zr = z + lane;
         for (int i = 0; i < max_rows; ++i, zr += 32) {
             if ((i & 7) == 0) {
@@ -135,7 +121,7 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
                 if ((e & (G - 1)) == 0) {
                     ext = tw = 0u;
                     if (i < rows) {
-                        ext = codes8(d, q_off, qlen, qrev, i - w + 8 * (G + r));
+                        ext = codes8(d.codes, d.nmask, q_off, qlen, qrev, i - w + 8 * (G + r));
                         const int ch = (e + r) >> 1;
                         if (ch << 4 < tlen) {
                             uint32_t x, nb;

@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps) group16_kernel(LaunchDesc d,
 void group16_tiles(TileTable& t) {
     const int w[] = {31, 63, 127, 255, 0x7FFFFFFF};
     t.n = 5;
+    t.by_rows = 1;
     for (int k = 0; k < 5; ++k) {
         t.width[k] = w[k]; t.lanes[k] = k < 4 ? 1 : 32; t.tile[k] = k < 4 ? 2 : 9;
         t.warp_batch[k] = 0; t.refill[k] = 1;

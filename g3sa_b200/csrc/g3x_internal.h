@@ -48,6 +48,8 @@ struct LaunchDesc {
     int32_t ring;          // lane-per-job kernel: 0, or the columns of its row-buffer ring
     int32_t pdl;           // class kernels: 1 = launched as a programmatic dependent of the
                            // class kernel before it on the stream (launch_class_kernel)
+    int32_t split;         // 1: the band kernel and the row-parallel kernel share the jobs by their
+                           // bands (band_window): each skips what is not its own
     int32_t retry;         // a seed-level retry wave: few of its n jobs, a device-side count
     int64_t n_bases;       // bases the planes hold: jobs reaching past them are refused
     int64_t step_limit;    // plain (rolling) kernel: per-job step bound, 0 = the default bound
@@ -59,6 +61,15 @@ __host__ __device__ __forceinline__ bool job_in_planes(const g3x_job_t& jb, int6
     return (int64_t)jb.q_off + jb.qlen <= n_bases && (int64_t)jb.t_off + jb.tlen <= n_bases;
 }
 
+// Who runs a job when a launch's jobs are split: the band kernel with the narrowest window of 256,
+// 512 or 1024 columns that holds the job's band (2 w + 2 entries, w the clamped width) while its
+// scores stay below 2^21, else (0) the row-parallel kernel.
+__host__ __device__ __forceinline__ int band_window(int32_t w, int32_t qlen, int32_t h0, int32_t max_sc) {
+    if ((int64_t)qlen * max_sc + (h0 > 0 ? h0 : 0) >= (1 << 21)) return 0;
+    const int need = 2 * w + 2;
+    return need <= 256 ? 256 : need <= 512 ? 512 : need <= 1024 ? 1024 : 0;
+}
+
 // Tile configurations by job width class (ascending width; the last class is unbounded).
 constexpr int kMaxBuckets = 8;
 struct TileTable {
@@ -68,6 +79,7 @@ struct TileTable {
     int32_t tile[kMaxBuckets];
     int32_t warp_batch[kMaxBuckets];
     int32_t refill[kMaxBuckets];
+    int32_t by_rows = 0;          // 1: classes of the group kernel, sorted by rows alone
 };
 
 // The width classes a new context starts with (and the no-alloc entry point always uses): each
@@ -249,7 +261,6 @@ int launch_band(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream)
 void group16_tiles(TileTable& t);
 int launch_group16(const LaunchDesc& d, const ScoreParams& sp, int32_t* misfit, int32_t* misfits,
                    cudaStream_t stream);
-size_t band_smem_per_warp(int qcap);
 size_t lane2_smem_per_warp(int qcap);
 size_t lane16_smem_per_warp(int qcap);
 size_t lane_ring_smem_per_warp(int ring);

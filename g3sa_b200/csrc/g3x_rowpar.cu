@@ -270,6 +270,11 @@ __global__ void __launch_bounds__(128) rowpar_kernel(LaunchDesc d, ScoreParams s
                 }
                 if (slot >= n) { exhausted = true; break; }
                 const int job = order ? order[slot] : slot;
+                if (d.split) {                 // the band kernel's
+                    const g3x_job_t jb = d.jobs[job];
+                    const int32_t w = clamp_w(jb.w, jb.qlen, sp.max_sc, sp.end_bonus, sp.o_del, sp.e_del, sp.o_ins, sp.e_ins);
+                    if (band_window(w, jb.qlen, jb.h0, sp.max_sc)) continue;
+                }
                 StagedJob sj;
                 uint32_t prof_lo[5], prof_hi[5];
                 score_pools(sp, prof_lo, prof_hi);

@@ -110,7 +110,8 @@ __global__ void scatter_kernel(const int32_t* __restrict__ bin, int n, int32_t* 
     order[at] = job_at(k, subset);
 }
 
-// Global-alignment jobs: the band class, then rows (four bins per doubling) and the widest row.
+// Global-alignment jobs: the band class, then rows (the groups' classes), or rows (four bins per
+// doubling) and the widest row (the lane kernel's).
 __global__ void pair_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int classes, int32_t* __restrict__ bin,
                                 int32_t* __restrict__ hist) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,10 +120,10 @@ __global__ void pair_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int c
     const int w = min(max(jb.w, 0), (int)max(jb.qlen, jb.tlen));
     int c = 0;
     while (c < classes && 2 * w + 1 > 16 << c) ++c;
-    int rb = (int)((16.0f - log2f(1.0f + (float)jb.tlen)) * (kSchedRowBins / 16.0f));
-    rb = min(max(rb, 0), kSchedRowBins - 1);
+    const float lr = log2f(1.0f + (float)jb.tlen);
+    const int rb = min(max((int)((16.0f - lr) * (kSchedRowBins / 16.0f)), 0), kSchedRowBins - 1);
     const int wb = kSchedWidthBins - 1 - min((min((int)jb.qlen, 2 * w + 1) + 7) >> 3, kSchedWidthBins - 1);
-    const int bn = c * kLevels + rb * kSchedWidthBins + wb;
+    const int bn = c * kLevels + (c < classes ? row_level(lr) : rb * kSchedWidthBins + wb);
     bin[k] = bn;
     sched_count(hist, bn);
 }

@@ -13,7 +13,8 @@
 //           (a z-drop on an unrelated target), and by how much further; its error on jobs that
 //           run to their end leaves them in length order, which is already near the true order
 //           for them.  Continuous, so jobs of equal predicted rows stay together;
-//   width : eight-column blocks of the widest row min(qlen, 2w' + 1), wider first.
+//   width : eight-column blocks of the widest row min(qlen, 2w' + 1), wider first (the group
+//           kernels' classes: finer row bins instead).
 #pragma once
 #include <math.h>
 #include "g3x_core.h"
@@ -24,6 +25,14 @@ namespace g3x {
 constexpr int kSchedRowBins = 64, kSchedWidthBins = 32;
 constexpr float kLearnedSlack = 1.0f;   // log2 rows the learned correction must exceed
 static_assert(kSchedRowBins * kSchedWidthBins == kSchedLevels, "key layout");
+
+// Row bins alone, 128 per doubling: for kernels whose row takes the same time whatever its width, so
+// that only the row count matters of what runs together (the group kernels' warps take their
+// jobs at once and wait for the longest).
+__device__ __forceinline__ int row_level(float log2_rows) {
+    const int rb = (int)((16.0f - log2_rows) * (kSchedLevels / 16.0f));
+    return rb < 0 ? 0 : (rb >= kSchedLevels ? kSchedLevels - 1 : rb);
+}
 
 // has_pred: the learned schedule, with the model's correction `pred` for this job.
 __device__ __forceinline__ int sched_key(const g3x_job_t& jb, const ScoreParams& sp, const TileTable& tt,
@@ -48,6 +57,7 @@ __device__ __forceinline__ int sched_key(const g3x_job_t& jb, const ScoreParams&
     }
     float lr = log2f(1.0f + (float)jb.tlen);
     if (has_pred) lr += fminf(pred + kLearnedSlack, 0.0f);
+    if (tt.by_rows || tt.lanes[b] == 32) return b * kSchedLevels + row_level(lr);
     int rb = (int)((16.0f - lr) * (kSchedRowBins / 16.0f));
     rb = rb < 0 ? 0 : (rb >= kSchedRowBins ? kSchedRowBins - 1 : rb);
     int wb = (wide + 7) >> 3;

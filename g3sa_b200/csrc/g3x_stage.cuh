@@ -127,6 +127,21 @@ __device__ __forceinline__ uint64_t nibbles16(uint32_t x, uint32_t nb) {
     return t | (n << 2);
 }
 
+// Codes of positions c .. c + 7 of a sequence as nibbles (nibbles16), 0 outside [0, len).
+__device__ __forceinline__ uint32_t codes8(const uint32_t* __restrict__ codes, const uint32_t* __restrict__ nmask,
+                                           uint32_t off, int len, bool rev, int c) {
+    const int ch = c >> 4, sh = (c & 15) << 2;
+    uint64_t v[2] = {0, 0};
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (ch + u >= 0 && (ch + u) << 4 < len && (u == 0 || sh > 32)) {
+            uint32_t x, nb;
+            load16(codes, nmask, off, len, ch + u, rev, x, nb);
+            v[u] = nibbles16(x, nb);
+        }
+    return (uint32_t)(v[0] >> sh) | (sh > 32 ? (uint32_t)(v[1] << (64 - sh)) : 0u);
+}
+
 // Chunks 0 .. nch-1 of the calling lane's own query as 4-bit codes into its column of a
 // lane-interleaved word array (chunk ch in words 2ch and 2ch+1, word k of lane L at
 // qn[k * 32 + L]).  The lanes of a refill wave each stage their own job at the same time, four
