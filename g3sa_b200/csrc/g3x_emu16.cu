@@ -36,7 +36,7 @@ uint8_t base_at(const uint8_t* u8, uint32_t off, int len, int k, bool rev) {
     return c < 4 ? c : 4;
 }
 
-template <bool kSym>
+template <bool kSym, bool kCells>
 int run_job(const g3x_job_t& jb, const uint8_t* u8, const ScoreParams& sp, const uint2* pools,
             const uint4* ge, g3x_ext_t* out, int32_t* cells) {
     JobConst c;
@@ -73,8 +73,7 @@ int run_job(const g3x_job_t& jb, const uint8_t* u8, const ScoreParams& sp, const
     J.job = 0;
     J.qlen = c.qlen; J.tlen = c.tlen; J.w = c.w; J.h0 = c.h0;
     J.t_off = jb.t_off; J.trev = trev;
-    commit_init(J.K, c);
-    J.beg = 0; J.end = c.qlen;
+    l16::start_job(J, c);
     while (!J.K.stop) {
         const int32_t i = J.K.next;
         J.tx = J.tn = 0;
@@ -92,11 +91,11 @@ int run_job(const g3x_job_t& jb, const uint8_t* u8, const ScoreParams& sp, const
         uint32_t mF, mL;
         // a one-block row elsewhere in the warp masks this lane's last block too: vary it
         const bool any_single = nblk == 1 || ((i * 2246822519u + (uint32_t)jb.t_off) >> 31);
-        l16::row_blocks<kSym>(P, 0, r, pc, ge, nblk, kmax, any_single, mF, mL);
-        l16::row_end(J, P, 0, r, sp, nonempty, mF, mL);
+        l16::row_blocks<kSym, kCells>(P, 0, r, pc, ge, nblk, kmax, any_single, mF, mL);
+        l16::row_end<kCells>(J, P, 0, r, sp, nonempty, mF, mL);
     }
     const Commit& K = J.K;
-    *out = g3x_ext_t{K.best, K.best_j + 1, K.best_i + 1, K.max_ie + 1, K.gscore, K.max_off};
+    *out = l16::finish_job(K);
     *cells = (int32_t)K.cells;
     return G3X_OK;
 }
@@ -122,8 +121,14 @@ extern "C" int g3x_emu16_extend(const g3x_job_t* jobs, int32_t n, const uint8_t*
     for (int32_t k = 0; k < n; ++k) {
         out[k] = g3x_ext_t{0, 0, 0, 0, 0, 0};
         cells[k] = 0;
-        status[k] = sym ? run_job<true>(jobs[k], u8, sp, pools, ge, &out[k], &cells[k])
-                        : run_job<false>(jobs[k], u8, sp, pools, ge, &out[k], &cells[k]);
+        status[k] = sym ? run_job<true, true>(jobs[k], u8, sp, pools, ge, &out[k], &cells[k])
+                        : run_job<false, true>(jobs[k], u8, sp, pools, ge, &out[k], &cells[k]);
+        // the form without cell counts: the same results
+        g3x_ext_t o2 = {0, 0, 0, 0, 0, 0};
+        int32_t none = 0;
+        const int st = sym ? run_job<true, false>(jobs[k], u8, sp, pools, ge, &o2, &none)
+                           : run_job<false, false>(jobs[k], u8, sp, pools, ge, &o2, &none);
+        if (st != status[k] || memcmp(&o2, &out[k], sizeof(o2)) != 0) status[k] = G3X_ERR_INTERNAL;
     }
     return G3X_OK;
 }

@@ -42,7 +42,7 @@ namespace g3x {
 
 size_t lane16_smem_per_warp(int qcap) { return l16::warp_bytes(qcap); }
 
-template <bool kSym>
+template <bool kSym, bool kCells>
 __global__ void __launch_bounds__(128) lane16_kernel(LaunchDesc d, ScoreParams sp) {
     pdl_trigger();
     using namespace l16;
@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(128) lane16_kernel(LaunchDesc d, ScoreParams s
                         J.qlen = c.qlen; J.tlen = c.tlen; J.w = c.w; J.h0 = c.h0;
                         J.t_off = jb.t_off;
                         J.trev = (jb.flags & G3X_JOB_TREV) != 0;
-                        commit_init(J.K, c);
-                        J.beg = 0; J.end = c.qlen;
+                        start_job(J, c);
                         J.tx = J.tn = 0;
                         J.pv = J.pm = 0;
                         if (c.tlen > 0) load16(d.codes, d.nmask, J.t_off, c.tlen, 0, J.trev, J.tx, J.tn);
@@ -175,17 +174,17 @@ __global__ void __launch_bounds__(128) lane16_kernel(LaunchDesc d, ScoreParams s
 
         // ---- the row's blocks: masked first block, middle blocks two at a time, masked last block ----
         uint32_t mF, mL;
-        row_blocks<kSym>(P, lane, r, pc, ge, nblk, kmax, any_single, mF, mL);
+        row_blocks<kSym, kCells>(P, lane, r, pc, ge, nblk, kmax, any_single, mF, mL);
 
         // ---- row end (ksw.cu:371-391) ----
         G3X_PHASE(2);
-        if (run) row_end(J, P, lane, r, sp, nonempty, mF, mL);
+        if (run) row_end<kCells>(J, P, lane, r, sp, nonempty, mF, mL);
         G3X_PHASE(3);
         if (active && J.K.stop) {
             const Commit& K = J.K;
-            d.out[J.job] = g3x_ext_t{K.best, K.best_j + 1, K.best_i + 1, K.max_ie + 1, K.gscore, K.max_off};
+            d.out[J.job] = finish_job(K);
             d.status[J.job] = G3X_OK;
-            if (d.cells) d.cells[J.job] = (int32_t)K.cells;
+            if (kCells) d.cells[J.job] = (int32_t)K.cells;
             if (d.rows) d.rows[J.job] = K.next;
             J.job = -1;
             busy += busy32; idle += kmax32 - busy32; busy32 = kmax32 = 0;
@@ -208,11 +207,11 @@ __global__ void __launch_bounds__(128) lane16_kernel(LaunchDesc d, ScoreParams s
     pdl_chain_end();
 }
 
-template <bool kSym>
+template <bool kSym, bool kCells>
 static int launch_lane16_t(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream) {
     const size_t wb = l16::warp_bytes(d.qmax);
     size_t max_smem = 0;
-    if (allow_max_smem(lane16_kernel<kSym>, &max_smem) != cudaSuccess) return G3X_ERR_CUDA;
+    if (allow_max_smem(lane16_kernel<kSym, kCells>, &max_smem) != cudaSuccess) return G3X_ERR_CUDA;
     if (wb > max_smem) return G3X_ERR_TOO_LONG;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return G3X_ERR_CUDA;
@@ -223,12 +222,12 @@ static int launch_lane16_t(const LaunchDesc& d, const ScoreParams& sp, cudaStrea
         const size_t smem = (size_t)wpb * wb;
         if (smem > max_smem) break;
         int per_sm = 0;
-        per_sm = resident_blocks(lane16_kernel<kSym>, 32 * wpb, smem);
+        per_sm = resident_blocks(lane16_kernel<kSym, kCells>, 32 * wpb, smem);
         if (per_sm * wpb >= best_warps) { best_warps = per_sm * wpb; best_wpb = wpb; best_blocks = per_sm; }
     }
     const size_t smem = (size_t)best_wpb * wb;
     const int blocks = d.blocks > 0 ? d.blocks : sms * (best_blocks > 0 ? best_blocks : 1);
-    if (launch_class_kernel(lane16_kernel<kSym>, blocks, 32 * best_wpb, smem, stream, d, sp) != cudaSuccess)
+    if (launch_class_kernel(lane16_kernel<kSym, kCells>, blocks, 32 * best_wpb, smem, stream, d, sp) != cudaSuccess)
         return G3X_ERR_CUDA;
     return G3X_OK;
 }
@@ -236,7 +235,9 @@ static int launch_lane16_t(const LaunchDesc& d, const ScoreParams& sp, cudaStrea
 // Gap opening and extension costs that agree between deletions and insertions (oe_del == oe_ins,
 // BWA's defaults) let the E step reuse the F step's max(M - oe, 0).
 int launch_lane16(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream) {
-    return sp.oe_del == sp.oe_ins ? launch_lane16_t<true>(d, sp, stream) : launch_lane16_t<false>(d, sp, stream);
+    const bool sym = sp.oe_del == sp.oe_ins;
+    if (d.cells) return sym ? launch_lane16_t<true, true>(d, sp, stream) : launch_lane16_t<false, true>(d, sp, stream);
+    return sym ? launch_lane16_t<true, false>(d, sp, stream) : launch_lane16_t<false, false>(d, sp, stream);
 }
 
 }  // namespace g3x

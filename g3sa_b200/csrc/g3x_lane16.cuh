@@ -33,6 +33,13 @@
 // beg > 0 as ksw.cu:344-345 sets it) comes out right.  The last block keeps the words right of
 // column end as they were (the band can grow back into them, ksw.cu:390-391), and leaves
 // columns >= end out of the row maximum.
+//
+// beg to the block only.  Since dead columns compute zeros, nothing but the cell count needs the
+// exact beg of the trim: it is kept as the first column of a block with a non-zero word (moved on by
+// a block when the row's first block comes out all zero), which spares the column search of the
+// trim.  h1 = H(i, -1) (ksw.cu:342-345) asks whether beg is 0, but while it is positive column 0
+// holds it and the trim stays at 0, and once it is 0 it stays 0.  kCells: the exact beg, for batches
+// that ask for their cell counts.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -294,8 +301,9 @@ G3X_HD void block_mid2(const Planes& P, int at, int32_t kb, bool second, RowStat
 }
 
 // The first block of a row with two or more blocks: the words left of beg are zeroed on load.
-// Returns the columns of the block at or right of beg whose new H or E word is non-zero.
-template <bool kSym>
+// Returns the columns of the block at or right of beg whose new H or E word is non-zero (without
+// kCells: non-zero when there is any).
+template <bool kSym, bool kCells>
 G3X_HD uint32_t block_first(const Planes& P, int at, int32_t kb, RowState& r, const PairConst& pc,
                             const uint4* ge) {
     const int32_t jb = kb << 3;
@@ -308,6 +316,7 @@ G3X_HD uint32_t block_first(const Planes& P, int at, int32_t kb, RowState& r, co
     P.H[at] = make_uint4(nh[0], nh[1], nh[2], nh[3]);
     P.E[at] = make_uint4(ne[0], ne[1], ne[2], ne[3]);
     block_max(h2, kb, r);
+    if (!kCells) return nh[0] | nh[1] | nh[2] | nh[3] | ne[0] | ne[1] | ne[2] | ne[3];
     return nonzero_mask(nh, ne, 0xFFu << (r.beg - jb));
 }
 
@@ -400,7 +409,7 @@ struct LaneJob {
     int32_t qlen, tlen, w, h0;
     uint32_t t_off;
     int32_t trev;
-    Commit K;
+    Commit K;                // best_j holds the best cell's diagonal, row - column (see finish_job)
     int32_t beg, end;        // band of the next row before the clamps of ksw.cu:338-340
     uint32_t tx, tn;         // target chunk K.next >> 4: 2-bit codes and N bits
     uint64_t pv, pm;         // the plane words of the next chunk (kernel prefetch)
@@ -436,34 +445,48 @@ G3X_HD void row_begin(const LaneJob& J, const ScoreParams& sp, const uint2* pool
     r.key = 0;
 }
 
+// No to-end score in a row: below gscore's start.
+constexpr int32_t kNoGscore = -2;
+
+G3X_HD void start_job(LaneJob& J, const JobConst& c) {
+    commit_init(J.K, c);
+    J.K.best_j = 0;                                     // diagonal of (-1, -1)
+    J.beg = 0;
+    J.end = c.qlen;
+}
+
+G3X_HD g3x_ext_t finish_job(const Commit& K) {
+    return g3x_ext_t{K.best, K.best_i - K.best_j + 1, K.best_i + 1, K.max_ie + 1, K.gscore, K.max_off};
+}
+
 // The row bookkeeping of ksw.cu:372-386 (the same as commit_row) with selects in place of
-// branches: to-end score, cell count, new maximum or z-drop, last row.
+// branches: to-end score, cell count, new maximum or z-drop, last row.  d.gval is kNoGscore in a row
+// without a to-end score; d.mj counts only when d.m > 0.
+template <bool kCells>
 G3X_HD void commit_row_sel(Commit& k, const JobConst& c, const RowDone& d) {
     const int32_t i = k.next;
-    // ksw.cu:372-375 for gval >= 0 (gval -1: no to-end score this row); gscore starts at -1 and
-    // only grows, so it is the running maximum of gval, and max_ie moves to i where gval >= 0
-    // reaches it
-    k.max_ie = d.gval >= (k.gscore > 0 ? k.gscore : 0) ? i : k.max_ie;
+    k.max_ie = d.gval >= k.gscore ? i : k.max_ie;                            // ksw.cu:372-375
     k.gscore = d.gval > k.gscore ? d.gval : k.gscore;
-    k.cells += d.ncells;
+    if (kCells) k.cells += d.ncells;
     k.next = i + 1;
     const bool up = d.m > k.best;                                            // ksw.cu:377-379
-    const int32_t di = i - k.best_i, dj = d.mj - k.best_j;                   // ksw.cu:380-386
-    const int32_t drop = di > dj ? k.best - d.m - (di - dj) * c.e_del : k.best - d.m - (dj - di) * c.e_ins;
-    const bool zstop = !up && c.zdrop > 0 && drop > c.zdrop;
-    const int32_t off = abs(d.mj - i);
-    k.max_off = up ? (off > k.max_off ? off : k.max_off) : k.max_off;
+    const int32_t dg = i - d.mj, t = dg - k.best_j;                          // ksw.cu:380-386
+    const int32_t gd = t * c.e_del, gi = -t * c.e_ins;                       // (never for a new maximum)
+    const bool zstop = k.best - d.m - (gd > gi ? gd : gi) > (c.zdrop > 0 ? c.zdrop : 0x7FFFFFFF);
+    const int32_t off = up ? abs(dg) : 0;
+    k.max_off = off > k.max_off ? off : k.max_off;
     k.best = d.m > k.best ? d.m : k.best;
     k.best_i = up ? i : k.best_i;
-    k.best_j = up ? d.mj : k.best_j;
+    k.best_j = up ? dg : k.best_j;
     k.stop = d.m == 0 || zstop || k.next >= c.tlen;                         // ksw.cu:376, the row loop
 }
 
 // Row end (ksw.cu:371-391) for a running lane: column end's words, the row's bookkeeping, and
 // the band of the next row.  mF: the columns >= beg of the row's first block with a non-zero new
-// word (rows of two or more blocks); mL: those up to column end of its last block.  The first
-// non-zero column from beg and the last one back from end are almost always found in them; the
-// row buffer is read only when not.
+// word (rows of two or more blocks; without kCells any non-zero value for some); mL: those up to
+// column end of its last block.  The first non-zero column from beg and the last one back from end
+// are almost always found in them; the row buffer is read only when not.
+template <bool kCells>
 G3X_HD void row_end(LaneJob& J, const Planes& P, int lane, const RowState& r, const ScoreParams& sp,
                     bool nonempty, uint32_t mF, uint32_t mL) {
     const int32_t beg = r.beg, end = r.end;
@@ -476,25 +499,29 @@ G3X_HD void row_end(LaneJob& J, const Planes& P, int lane, const RowState& r, co
     }
     RowDone rd;
     rd.m = r.key >> 16;
-    const int32_t mj = max_col(P, lane, r.key, beg, end);
-    rd.mj = rd.m > 0 ? mj : -1;
-    rd.gval = (nonempty ? end : beg) == J.qlen ? r.h1 : -1;
+    rd.mj = max_col(P, lane, r.key, beg, end);
+    rd.gval = (nonempty ? end : beg) == J.qlen ? r.h1 : kNoGscore;
     rd.ncells = nonempty ? end - beg : 0;
-    commit_row_sel(J.K, job_const(J, sp), rd);
+    commit_row_sel<kCells>(J.K, job_const(J, sp), rd);
     if (J.K.stop) return;
     // (a row that does not stop has a non-empty band)
     // ksw.cu:388-389: the first column of [beg, end) whose H or E word is non-zero, else end
-    const uint32_t mk = jb0 < jbl ? mF : (mL & (0xFFu << (beg - jb0)) & (0xFFu >> (kLB - (end - jb0))));
-    int32_t nb = end;
-    if (mk) {
-        nb = jb0 + ffs32(mk) - 1;
+    int32_t nb;
+    if (!kCells) {
+        nb = jb0 < jbl && mF == 0 ? jb0 + kLB : jb0;      // (to the block: see above)
     } else {
-        for (int32_t b = jb0 + kLB; b < end; b += kLB) {
-            uint32_t m2 = nonzero_cols(P, b, lane);
-            if (end - b < kLB) m2 &= 0xFFu >> (kLB - (end - b));
-            if (m2) {
-                nb = b + ffs32(m2) - 1;
-                break;
+        const uint32_t mk = jb0 < jbl ? mF : (mL & (0xFFu << (beg - jb0)) & (0xFFu >> (kLB - (end - jb0))));
+        nb = end;
+        if (mk) {
+            nb = jb0 + ffs32(mk) - 1;
+        } else {
+            for (int32_t b = jb0 + kLB; b < end; b += kLB) {
+                uint32_t m2 = nonzero_cols(P, b, lane);
+                if (end - b < kLB) m2 &= 0xFFu >> (kLB - (end - b));
+                if (m2) {
+                    nb = b + ffs32(m2) - 1;
+                    break;
+                }
             }
         }
     }
@@ -502,16 +529,16 @@ G3X_HD void row_end(LaneJob& J, const Planes& P, int lane, const RowState& r, co
     int32_t last = nb - 1;
     if (end_next && r.h1 != 0) {
         last = end;
-    } else if (nb <= jbl + kLB - 1) {
-        const uint32_t ml = nb > jbl ? mL & (0xFFu << (nb - jbl)) : mL;
+    } else if (!kCells || nb <= jbl + kLB - 1) {
+        const uint32_t ml = kCells && nb > jbl ? mL & (0xFFu << (nb - jbl)) : mL;
         if (ml) {
-            last = jbl + 31 - clz32(ml);
+            last = jbl + msb32(ml);
         } else {
             for (int32_t b = jbl - kLB; b >= (nb & ~(kLB - 1)); b -= kLB) {
                 uint32_t m2 = nonzero_cols(P, b, lane);
-                if (b < nb) m2 &= 0xFFu << (nb - b);
+                if (kCells && b < nb) m2 &= 0xFFu << (nb - b);
                 if (m2) {
-                    last = b + 31 - clz32(m2);
+                    last = b + msb32(m2);
                     break;
                 }
             }
@@ -528,13 +555,13 @@ G3X_HD void row_end(LaneJob& J, const Planes& P, int lane, const RowState& r, co
 // number of them is left for the warp), the last (masked).  Returns the first block's and the
 // last block's non-zero column masks for row_end in mF, mL.  any_single: some lane of the warp
 // has a one-block row (nblk == 1).
-template <bool kSym>
+template <bool kSym, bool kCells>
 G3X_HD void row_blocks(const Planes& P, int lane, RowState& r, const PairConst& pc, const uint4* ge,
                        int nblk, int kmax, bool any_single, uint32_t& mF, uint32_t& mL) {
     mF = mL = 0;
     const int32_t kb0 = r.beg >> 3;                 // block index of the first block
     const int at0 = (kb0 << 5) + lane;              // its uint4 index in the lane-interleaved planes
-    if (nblk > 1) mF = block_first<kSym>(P, at0, kb0, r, pc, ge);
+    if (nblk > 1) mF = block_first<kSym, kCells>(P, at0, kb0, r, pc, ge);
     int k = 1, at = at0 + 32;
     for (; k + 1 < kmax - 1; k += 2, at += 64)
         if (k < nblk - 1) block_mid2<kSym>(P, at, kb0 + k, k + 1 < nblk - 1, r, pc);
