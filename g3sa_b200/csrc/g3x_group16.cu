@@ -14,8 +14,7 @@
 // is a max-plus prefix over the group (log2 G shuffles of the blocks' outgoing F, decaying by
 // 8 e_ins per lane); H of the column left of a block comes from the lane before it by one
 // shuffle; the row maximum with its last column is one max over (H << 16 | column) keys; and the
-// band trims (ksw.cu:388-391) take the first and last lane of a ballot over the lanes' non-zero
-// column masks.  Band edges follow g3x_lane16.cuh: columns left of beg hold zeros (the words the
+// trim of end (ksw.cu:390-391) takes the last lane of a ballot over the lanes' non-zero column masks.  Band edges follow g3x_lane16.cuh: columns left of beg hold zeros (the words the
 // band clamp cuts off are zeroed), columns right of end keep their words, column end gets
 // {H(i, end-1), 0}, which the shifted H words of its block hold already.
 //
@@ -98,11 +97,12 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
     uint32_t H[4] = {0u, 0u, 0u, 0u}, E[4] = {0u, 0u, 0u, 0u};
     uint32_t qw = 0, tw = 0;      // query codes of the block; target codes of rows 8 (r + G c) ..
     uint2 pl = pools[0];          // score pools of row i
-    // row i - 1: (maximum << 16 | its last column), its to-end score, its band, and its first and
-    // last lanes with non-zero columns with their masks
-    int32_t key = kNoRow, gval = kNoGscore, end = 0;
-    int fl = 0, ll = 0;
-    uint32_t nzf = 1u, nzl = 1u;
+    // row i - 1: (maximum << 16 | its last column), its to-end score, and its last lane with
+    // non-zero columns with their mask
+    int32_t key = kNoRow, gval = kNoGscore;
+    int ll = 0;
+    uint32_t nzl = 1u;
+    int32_t beg = 0;              // kept for the cell counts only (see g3x_lane16.cuh)
     bool exhausted = false, all_idle = true;
     int32_t iters = 0;
     unsigned long long rows = 0;
@@ -229,9 +229,8 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                             E[p] = 0u;
                         }
                         // the band of row 0: all of [0, qlen)
-                        fl = gb; nzf = 1u;
                         ll = gb + 64; nzl = 1u;
-                        end = c.qlen;
+                        beg = 0;
                     }
                 }
                 // start the iteration anew: nothing is left of row i - 1, and a new job's blocks
@@ -248,11 +247,9 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
 
         // ---- the band of row i (ksw.cu:388-391, then 335-345) ----
         const int32_t cut = J.i - J.w;
-        const int32_t beg = max(8 * (fl - gb) + ffs32(nzf) - 1, cut);
-        end = min(min(8 * (ll - gb) + msb32(nzl) + 2, J.i + J.w + 1), J.qlen);
-        const int32_t h1 = beg == 0 ? max(J.hv, 0) : 0;
+        const int32_t end = min(min(8 * (ll - gb) + msb32(nzl) + 2, J.i + J.w + 1), J.qlen);
+        const int32_t h1 = cut <= 0 ? max(J.hv, 0) : 0;
         J.hv -= sp.e_del;
-        J.cells += max(end - beg, 0);
         const int h = max(min(end - col0, 8), -1) + 1;
         const uint4 lv = tab.left[h], rv = tab.right[h];
         const uint32_t left[4] = {lv.x, lv.y, lv.z, lv.w}, right[4] = {rv.x, rv.y, rv.z, rv.w};
@@ -279,16 +276,18 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
         }
         const uint32_t nz = nonzero_mask(H, E, upto);
         const unsigned bal = __ballot_sync(kAll, nz != 0u) & gmask;
-        fl = ffs32(bal) - 1;
         ll = msb32(bal);
-        nzf = __shfl_sync(kAll, nz, fl & 31);
         nzl = __shfl_sync(kAll, nz, ll & 31);
-        // to-end score: H(i, qlen - 1) is the H word of column qlen (used in its lane only); an
-        // empty row ends at beg with h1
+        if (d.cells) {
+            J.cells += max(end - max(beg, cut), 0);
+            const int fl = ffs32(bal) - 1;
+            beg = 8 * (fl - gb) + ffs32(__shfl_sync(kAll, nz, fl & 31)) - 1;
+        }
+        // to-end score: H(i, qlen - 1) is the H word of column qlen (used in its lane only)
         {
             const bool w2 = (J.qlen & 2) != 0;
             const int32_t v = (int32_t)prmt(w2 ? H[2] : H[0], w2 ? H[3] : H[1], J.qsel);
-            gval = max(beg, end) == J.qlen ? (beg < end ? v : h1) : kNoGscore;
+            gval = end == J.qlen ? v : kNoGscore;
         }
         // the column that the band clamp cuts off in row i + 1 (ksw.cu:338) becomes zero
         const int cc = cut - col0;
