@@ -23,9 +23,10 @@
 // wrapping and non-wrapping forms agree, and "subtract, 0 if not positive" of a non-negative
 // cell never wraps.  Longer queries get G3X_ERR_TOO_LONG.
 //
-// Jobs are sorted by segment count and target length (a device counting sort), so a warp's
-// eight jobs have about the same work; each of three launches (8, 16, 32 segments) takes its
-// class's range from a device counter.
+// Jobs are sorted by segment count and rows (a device counting sort), so a warp's eight jobs have
+// the same segments and about the same rows; each of three launches (8, 16, 32 segments) takes
+// its class's range from a device counter.  The second pass for the start positions (KSW_XSTART) has
+// its own sort and launches.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
@@ -39,7 +40,7 @@ namespace {
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kQuads = 8;                 // jobs per warp
 constexpr int kWarps = 4;                 // warps per block
-constexpr int kRowBins = 16;              // log2 of the target length
+constexpr int kRowBins = 128;             // rows, eight bins per doubling
 constexpr int kSegBins = 32;              // segments 1..32
 constexpr int kBins = kSegBins * kRowBins + 1;   // + the bin of rejected jobs (qlen 0 or > 256)
 constexpr int kNoScore = 0x10000;         // minsc / endsc when the flag is absent (ksw.cu:176-177)
@@ -330,12 +331,19 @@ __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen,
     return PassOut{gmax, te, qe};
 }
 
-template <int MAXSEG>
+// SECOND false: the first pass of every job.  SECOND: the start positions (ksw.cu:286-291) of the jobs
+// that want them, sorted anew by the segments and rows of their second pass: the query prefix
+// 0..qe and the target with its prefix 0..te reversed, stopping at the first score.  (Run by the warp
+// that ran the first pass, the second passes of eight jobs of one segment count have eight
+// segment counts, and each of a segment's steps ran once for every few of them: 15.8 of 32 lanes active
+// and 3.0 ms more on 200k windows.)
+template <int MAXSEG, bool SECOND>
 __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) sw_kernel(SwDesc d) {
     constexpr int QMAX = 8 * MAXSEG;
     __shared__ __align__(16) uint8_t qcodes[kWarps][kQuads][QMAX];
     __shared__ uint32_t snap[kWarps][MAXSEG * 32];
     __shared__ uint2 tab[5];
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane >> 2, p = lane & 3;
     if (threadIdx.x < 5) tab[threadIdx.x] = make_uint2(d.tab[2 * threadIdx.x], d.tab[2 * threadIdx.x + 1]);
     __syncthreads();
@@ -361,73 +369,85 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
             int st = G3X_OK;
             if (qlen < 1) st = G3X_ERR_INVALID;     // the reference reads before its buffers
             else if (!job_in_planes(jb, d.n_bases)) st = G3X_ERR_INVALID;   // past the planes: unread
-            else if (qlen > QMAX || (subo && tlen > d.sub_stride)) st = G3X_ERR_TOO_LONG;
-            if (st != G3X_OK) {
+            else if (qlen > 8 * kSegBins || (subo && tlen > d.sub_stride)) st = G3X_ERR_TOO_LONG;
+            if (st != G3X_OK) {                     // (first pass only: the second takes none of them)
                 if (p == 0) {
                     d.out[job] = g3x_swr_t{0, -1, -1, -1, -1, -1, -1};
                     d.status[job] = st;
                 }
             } else {
                 live = true;
-                const bool qrev = (jb.flags & G3X_JOB_QREV) != 0;
-                for (int pos = p; pos < qlen; pos += 4) qc[pos] = (uint8_t)base_at(d.codes, d.nmask, jb.q_off, qlen, pos, qrev);
             }
         }
-        __syncwarp();
-        const bool trev = live && (jb.flags & G3X_JOB_TREV) != 0;
+        const bool trev = live && (jb.flags & G3X_JOB_TREV) != 0, qrev = live && (jb.flags & G3X_JOB_QREV) != 0;
         Rows rows;
         rows.off = live ? jb.t_off : 0u; rows.len = tlen; rows.rev = trev;
         rows.roff = 0u; rows.rlen = 0; rows.rrev = false; rows.flip = 0;
         rows.chunk = -1; rows.view = -1; rows.x = 0u; rows.nb = 0u;
-        uint32_t* sub = subo && live ? d.sub + (int64_t)job * d.sub_stride : nullptr;
-        int n_b = 0;
-        const PassOut r = sw_pass<MAXSEG>(d, live, qlen, tlen, [&](int pos) { return (uint32_t)qc[pos]; }, rows,
-                                          minsc, endsc, sub, &n_b, hm, tab, lane);
-        g3x_swr_t o{r.score, r.te, r.qe, -1, -1, -1, -1};
-        // second best: list entries more than ceil(score / max(mat)) rows from te (ksw.cu:249-256)
-        if (live && p == 0 && n_b > 0) {
-            const int c = (r.score + d.maxmat - 1) / d.maxmat, low = r.te - c, high = r.te + c;
-            for (int k = 0; k < n_b; ++k) {
-                const uint32_t v = sub[k];
-                const int e = (int)(v & 0xFFFFu), sc = (int)(v >> 16);
-                if ((e < low || e > high) && sc > o.score2) { o.score2 = sc; o.te2 = e; }
+        if constexpr (!SECOND) {
+            if (live)
+                for (int pos = p; pos < qlen; pos += 4) qc[pos] = (uint8_t)base_at(d.codes, d.nmask, jb.q_off, qlen, pos, qrev);
+            __syncwarp();
+            uint32_t* sub = subo && live ? d.sub + (int64_t)job * d.sub_stride : nullptr;
+            int n_b = 0;
+            const PassOut r = sw_pass<MAXSEG>(d, live, qlen, tlen, [&](int pos) { return (uint32_t)qc[pos]; }, rows,
+                                              minsc, endsc, sub, &n_b, hm, tab, lane);
+            g3x_swr_t o{r.score, r.te, r.qe, -1, -1, -1, -1};
+            // second best: list entries more than ceil(score / max(mat)) rows from te (ksw.cu:249-256)
+            if (live && p == 0 && n_b > 0) {
+                const int c = (r.score + d.maxmat - 1) / d.maxmat, low = r.te - c, high = r.te + c;
+                for (int k = 0; k < n_b; ++k) {
+                    const uint32_t v = sub[k];
+                    const int e = (int)(v & 0xFFFFu), sc = (int)(v >> 16);
+                    if ((e < low || e > high) && sc > o.score2) { o.score2 = sc; o.te2 = e; }
+                }
             }
-        }
-        // start positions (ksw.cu:286-291): the query prefix 0..qe and the target with its prefix
-        // 0..te reversed, stopping at the first score; kept when it finds the same score
-        const bool two = live && (d.xtra & G3X_KSW_XSTART) && !(subo && r.score < (d.xtra & 0xFFFF));
-        if (__any_sync(kFull, two)) {
-            const int lq = r.qe + 1, lt = r.te + 1;
-            Rows rows2 = rows;
-            rows2.chunk = -1; rows2.view = -1;
-            rows2.flip = two ? lt : 0;
-            rows2.rlen = lt;
-            if (!trev) { rows2.roff = rows.off; rows2.rrev = true; }
-            else { rows2.roff = rows.off + (uint32_t)(tlen - lt); rows2.rrev = false; }
-            const int qe1 = r.qe;
-            const PassOut rr = sw_pass<MAXSEG>(d, two, lq, tlen, [&](int pos) { return (uint32_t)qc[qe1 - pos]; },
-                                               rows2, kNoScore, r.score, nullptr, nullptr, hm, tab, lane);
-            if (two && rr.score == r.score) { o.tb = r.te - rr.te; o.qb = r.qe - rr.qe; }
-        }
-        if (live && p == 0) {
-            d.out[job] = o;
-            d.status[job] = G3X_OK;
+            if (live && p == 0) {
+                d.out[job] = o;
+                d.status[job] = G3X_OK;
+            }
+        } else {
+            int score = 0, te = -1, qe = 0;
+            if (live) { score = d.out[job].score; te = d.out[job].te; qe = d.out[job].qe; }
+            const int lq = live ? qe + 1 : 0, lt = te + 1;
+            if (live)
+                for (int pos = p; pos < lq; pos += 4) qc[pos] = (uint8_t)base_at(d.codes, d.nmask, jb.q_off, qlen, qe - pos, qrev);
+            __syncwarp();
+            rows.flip = lt;
+            rows.rlen = lt;
+            if (!trev) { rows.roff = rows.off; rows.rrev = true; }
+            else { rows.roff = rows.off + (uint32_t)(tlen - lt); rows.rrev = false; }
+            const PassOut rr = sw_pass<MAXSEG>(d, live, lq, tlen, [&](int pos) { return (uint32_t)qc[pos]; }, rows,
+                                               kNoScore, score, nullptr, nullptr, hm, tab, lane);
+            if (live && p == 0 && rr.score == score) {      // kept when it finds the same score
+                d.out[job].tb = te - rr.te;
+                d.out[job].qb = qe - rr.qe;
+            }
         }
         __syncwarp();
     }
+    pdl_chain_end();
 }
 
-// Sort bins: segment count descending, then target length descending (log2); the last bin
-// holds the jobs the kernels reject.
-__global__ void sw_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int32_t* __restrict__ bin,
+// Sort bins: segment count descending, then rows descending; the last bin holds the jobs the first
+// pass rejects, or (res set: the second pass) those without one -- refused ones and, under
+// KSW_XSUBO, scores below the threshold.
+__global__ void sw_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, const g3x_swr_t* __restrict__ res,
+                              const int32_t* __restrict__ status, int min_score, int32_t* __restrict__ bin,
                               int32_t* __restrict__ hist) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const g3x_job_t jb = jobs[k];
+    int qlen = jb.qlen, rows = jb.tlen;
+    if (res) {
+        const g3x_swr_t r = res[k];
+        qlen = status[k] == G3X_OK && r.score >= min_score ? r.qe + 1 : 0;
+        if (r.te >= 0) rows = r.te + 1;
+    }
     int b = kBins - 1;
-    if (jb.qlen >= 1 && jb.qlen <= 8 * kSegBins) {
-        const int slen = (jb.qlen + 7) >> 3;
-        const int rb = 31 - __clz((int)jb.tlen | 1);
+    if (qlen >= 1 && qlen <= 8 * kSegBins) {
+        const int slen = (qlen + 7) >> 3;
+        const int rb = (int)(log2f(1.0f + (float)rows) * 8.0f);
         b = (kSegBins - slen) * kRowBins + (kRowBins - 1 - min(rb, kRowBins - 1));
     }
     bin[k] = b;
@@ -436,27 +456,39 @@ __global__ void sw_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int32_t
 }
 
 // Exclusive scan of the bins (one block) and the three launches' ranges: 17-32 segments, 9-16,
-// and 1-8 together with the rejected bin.
-__global__ void sw_scan_kernel(const int32_t* __restrict__ hist, int32_t* __restrict__ cursor,
-                               int32_t* __restrict__ range, int n) {
+// and 1-8, in the first pass together with the rejected bin (with_last).
+__global__ void __launch_bounds__(1024) sw_scan_kernel(const int32_t* __restrict__ hist, int32_t* __restrict__ cursor,
+                                                       int32_t* __restrict__ range, int with_last) {
+    constexpr int kPer = (kBins + 1023) / 1024;
     __shared__ int32_t part[1024];
     const int t = threadIdx.x;
-    part[t] = t < kBins ? hist[t] : 0;
+    int32_t v[kPer], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        v[u] = t * kPer + u < kBins ? hist[t * kPer + u] : 0;
+        sum += v[u];
+    }
+    part[t] = sum;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
-        const int v = t >= o ? part[t - o] : 0;
+        const int x = t >= o ? part[t - o] : 0;
         __syncthreads();
-        part[t] += v;
+        part[t] += x;
         __syncthreads();
     }
-    if (t < kBins) cursor[t] = t ? part[t - 1] : 0;
+    int32_t at = part[t] - sum;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        if (t * kPer + u < kBins) cursor[t * kPer + u] = at;
+        at += v[u];
+    }
     __syncthreads();
     if (t == 0) {
-        const int b16 = (kSegBins - 16) * kRowBins, b8 = (kSegBins - 8) * kRowBins;
-        const int c16 = part[b16 - 1], c8 = part[b8 - 1];
+        const int c16 = cursor[(kSegBins - 16) * kRowBins], c8 = cursor[(kSegBins - 8) * kRowBins];
+        const int last = cursor[kBins - 1] + (with_last ? hist[kBins - 1] : 0);
         range[0] = 0;   range[1] = c16;
         range[2] = c16; range[3] = c8 - c16;
-        range[4] = c8;  range[5] = n - c8;
+        range[4] = c8;  range[5] = last - c8;
     }
 }
 
@@ -475,14 +507,48 @@ __global__ void sw_scatter_kernel(const int32_t* __restrict__ bin, int n, int32_
 
 uint32_t pack16(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; }
 
-template <int MAXSEG>
-int launch_class(const SwDesc& d0, const int32_t* range, int32_t* queue, int sms, cudaStream_t st) {
+template <int MAXSEG, bool SECOND>
+int launch_class(const SwDesc& d0, const int32_t* range, int32_t* queue, bool first, cudaStream_t st) {
     SwDesc d = d0;
     d.range = range;
     d.queue = queue;
-    const int per_sm = resident_blocks(sw_kernel<MAXSEG>, 32 * kWarps, 0);
-    sw_kernel<MAXSEG><<<sms * std::max(per_sm, 1), 32 * kWarps, 0, st>>>(d);
-    return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
+    auto kern = sw_kernel<MAXSEG, SECOND>;
+    const int per_sm = resident_blocks(kern, 32 * kWarps, 0);
+    // the classes of a pass run side by side: programmatic dependents of one another
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() * std::max(per_sm, 1)));
+    cfg.blockDim = dim3(32 * kWarps);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = first ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, d) == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;
+}
+
+// One pass over the jobs: sorted, then a launch per class.
+template <bool SECOND>
+int run_pass(const SwDesc& d, int32_t n, int32_t* buf, cudaStream_t st) {
+    int32_t* bin = buf;
+    int32_t* order = bin + n;
+    int32_t* hist = order + n;
+    int32_t* cursor = hist + kBins;
+    int32_t* range = cursor + kBins;      // 6 used, 8 kept
+    int32_t* queue = range + 8;           // 3 used, 4 kept
+    if (cudaMemsetAsync(hist, 0, sizeof(int32_t) * kBins, st) != cudaSuccess ||
+        cudaMemsetAsync(queue, 0, sizeof(int32_t) * 4, st) != cudaSuccess)
+        return G3X_ERR_CUDA;
+    const int min_score = (d.xtra & G3X_KSW_XSUBO) ? d.xtra & 0xFFFF : -1;
+    const int tb = 256, nb = (n + tb - 1) / tb;
+    sw_bin_kernel<<<nb, tb, 0, st>>>(d.jobs, n, SECOND ? d.out : nullptr, d.status, min_score, bin, hist);
+    sw_scan_kernel<<<1, 1024, 0, st>>>(hist, cursor, range, SECOND ? 0 : 1);
+    sw_scatter_kernel<<<nb, tb, 0, st>>>(bin, n, cursor, order);
+    if (cudaPeekAtLastError() != cudaSuccess) return G3X_ERR_CUDA;
+    int rc;
+    if ((rc = launch_class<32, SECOND>(d, range, queue, true, st))) return rc;
+    if ((rc = launch_class<16, SECOND>(d, range + 2, queue + 1, false, st))) return rc;
+    return launch_class<8, SECOND>(d, range + 4, queue + 2, false, st);
 }
 
 }  // namespace
@@ -521,24 +587,10 @@ extern "C" int g3x_ksw_align2_batch(g3x_ctx* ctx, const g3x_score_t* score, cons
         }
         s.cap = cap; s.sub_cap = sub_cap;
     }
-    int32_t* bin = s.buf;
-    int32_t* order = bin + n;
-    int32_t* hist = order + n;
-    int32_t* cursor = hist + kBins;
-    int32_t* range = cursor + kBins;      // 6 used, 8 kept
-    int32_t* queue = range + 8;           // 3 used, 4 kept
     const cudaStream_t st = (cudaStream_t)stream;
-    if (cudaMemsetAsync(hist, 0, sizeof(int32_t) * kBins, st) != cudaSuccess ||
-        cudaMemsetAsync(queue, 0, sizeof(int32_t) * 4, st) != cudaSuccess)
-        return G3X_ERR_CUDA;
-    const int tb = 256, nb = (n + tb - 1) / tb;
-    sw_bin_kernel<<<nb, tb, 0, st>>>(d_jobs, n, bin, hist);
-    sw_scan_kernel<<<1, 1024, 0, st>>>(hist, cursor, range, n);
-    sw_scatter_kernel<<<nb, tb, 0, st>>>(bin, n, cursor, order);
-    if (cudaPeekAtLastError() != cudaSuccess) return G3X_ERR_CUDA;
     SwDesc d;
     memset(&d, 0, sizeof(d));
-    d.jobs = d_jobs; d.codes = d_codes; d.nmask = d_nmask; d.order = order;
+    d.jobs = d_jobs; d.codes = d_codes; d.nmask = d_nmask; d.order = s.buf + n;
     d.out = d_out; d.status = d_status;
     d.sub = subo ? s.sub : nullptr;
     d.sub_stride = subo ? std::max(max_tlen, 1) : 0;
@@ -558,9 +610,6 @@ extern "C" int g3x_ksw_align2_batch(g3x_ctx* ctx, const g3x_score_t* score, cons
     d.dec0 = 0x10000u + d.step;
     d.peins = pack16(sp.e_ins);
     d.nstep = pack16(-d.carry_e);
-    int sms = 0;
-    sms = sm_count();
-    if ((rc = launch_class<32>(d, range, queue, sms, st))) return rc;
-    if ((rc = launch_class<16>(d, range + 2, queue + 1, sms, st))) return rc;
-    return launch_class<8>(d, range + 4, queue + 2, sms, st);
+    if ((rc = run_pass<false>(d, n, s.buf, st))) return rc;
+    return (xtra & G3X_KSW_XSTART) ? run_pass<true>(d, n, s.buf, st) : G3X_OK;
 }
