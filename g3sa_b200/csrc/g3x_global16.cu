@@ -19,9 +19,10 @@
 // keeps H(i, -1) of the row that will need it as its diagonal.  Cells right of the query need no
 // mask: F flows right, E stays in its column.  E entering at index 2w is 0.
 //
-// A cell's direction is four bits: E beats M, F beats both, E and F continue (ksw.cu:753-776), each
-// the difference of a maximum and one of its operands, formed by multiply-adds (the bias keeps
-// both halves non-negative, so one 32-bit subtraction serves both) and clipped to 0 or 1.  A
+// A cell's direction is four bits: H is not M, H is not E, E and F continue (ksw.cu:753-776: M
+// before E before F), each the difference of a maximum and one of its operands, formed by
+// multiply-adds (the bias keeps both halves non-negative, so one 32-bit subtraction serves both)
+// and clipped to 0 or 1.  A
 // lane's eight cells make one word, a warp's row one 128-byte line of scratch.  The backtrack
 // (ksw.cu:783-806) stays on one index while it moves diagonally, so the group reads G rows of that
 // index at a time and takes the run of matches up to the first gap from a ballot; gaps go cell by
@@ -174,10 +175,9 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
             uint32_t dir = 0u;
 #pragma unroll
             for (int p = 3; p >= 0; --p) {
-                const uint32_t me = __vimax3_s16x2(M[p], E[p], E[p]);
                 const uint32_t h = __vimax3_s16x2(M[p], E[p], F[p]);
                 const uint32_t one = 0x00010001u;
-                const uint32_t b0 = __vimin3_u16x2(M[p] * minus + me, one, one), b1 = __vimin3_u16x2(me * minus + h, one, one);
+                const uint32_t b0 = __vimin3_u16x2(M[p] * minus + h, one, one), b1 = __vimin3_u16x2(E[p] * minus + h, one, one);
                 const uint32_t b2 = __vimin3_u16x2(Td[p] * minus + En[p], one, one);
                 const uint32_t b3 = __vimin3_u16x2(T[p] * minus + F[p + 1], one, one);
                 dir = dir * 16u + (b0 + 2u * b1 + 4u * b2 + 8u * b3);
@@ -228,8 +228,8 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
             const int cells = min(min(i, k) + 1, which ? 1 : G);  // a gap goes on cell by cell
             uint32_t nib = 0u;
             if (go && !bad && r < cells) nib = (z[(int64_t)(i - r) * 32 + gb + (dk >> 3)] >> ((dk & 7) << 2)) & 0xFu;
-            // the operation at the cell: from H (bit 1 over bit 0), or the gap going on or not
-            const int o = which == 0 ? ((nib & 2u) ? 2 : (int)(nib & 1u)) : (nib >> (which + 1)) & 1u ? which : 0;
+            // the operation at the cell: from H (M, else E, else F), or the gap going on or not
+            const int o = which == 0 ? ((nib & 1u) ? 1 + (int)(nib >> 1 & 1u) : 0) : (nib >> (which + 1)) & 1u ? which : 0;
             const unsigned gap = __ballot_sync(kAll, go && r < cells && o != 0) & gmask;
             const int at = gap ? __ffs(gap) - 1 : 0;
             const int og = __shfl_sync(kAll, o, at);
