@@ -193,18 +193,21 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
             d.n_cigar[job] = full || bad ? 0 : n;
             int32_t stj = full ? G3X_ERR_TOO_LONG : bad ? G3X_ERR_INTERNAL : G3X_OK;
             if (d.nm && stj == G3X_OK) {
-                // the query from its codes in shared memory, the target from the planes 16 codes at a time
+                // the query from its codes in shared memory, the target from the planes
                 int cy = -1;
-                uint32_t ty = 0, tyn = 0;
-                auto qcode = [&](int p) -> uint32_t {
-                    const uint32_t nib = (qn[(p >> 3) * 32 + lane] >> ((p & 7) << 2)) & 0xFu;
-                    return (nib & 4u) ? 4u : nib;
+                uint64_t vy = 0;
+                auto qchunk = [&](int c) -> uint64_t {
+                    return plain_nibbles((uint64_t)qn[2 * c * 32 + lane] | (uint64_t)qn[(2 * c + 1) * 32 + lane] << 32);
                 };
-                auto tcode = [&](int p) -> uint32_t {
-                    if ((p >> 4) != cy) { cy = p >> 4; load16(d.codes, d.nmask, t_off, tlen, cy, trev, ty, tyn); }
-                    return ((tyn >> (p & 15)) & 1u) ? 4u : (ty >> ((p & 15) << 1)) & 3u;
+                auto tchunk = [&](int c) -> uint64_t {
+                    if (c != cy) {
+                        uint32_t x, nb;
+                        load16(d.codes, d.nmask, t_off, tlen, cy = c, trev, x, nb);
+                        vy = plain_nibbles(nibbles16(x, nb));
+                    }
+                    return vy;
                 };
-                if (!write_nm_md(d, job, flags, cg, n, qcode, tcode)) stj = G3X_ERR_TOO_LONG;
+                if (!write_nm_md(d, job, flags, cg, n, qchunk, tchunk)) stj = G3X_ERR_TOO_LONG;
             } else if (d.nm) {
                 d.nm[job] = 0;
                 d.md[(int64_t)job * d.md_stride] = 0;

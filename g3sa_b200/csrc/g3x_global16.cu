@@ -257,16 +257,24 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
                 int32_t st = full ? G3X_ERR_TOO_LONG : bad ? G3X_ERR_INTERNAL : G3X_OK;
                 if (d.nm && st == G3X_OK) {
                     int cq = -1, ct = -1;
-                    uint32_t xq = 0, nq = 0, xt = 0, nt = 0;
-                    auto qcode = [&](int p) -> uint32_t {
-                        if ((p >> 4) != cq) { cq = p >> 4; load16(d.codes, d.nmask, q_off, qlen, cq, qrev, xq, nq); }
-                        return ((nq >> (p & 15)) & 1u) ? 4u : (xq >> ((p & 15) << 1)) & 3u;
+                    uint64_t vq = 0, vt = 0;
+                    auto qchunk = [&](int c) -> uint64_t {
+                        if (c != cq) {
+                            uint32_t x, nb;
+                            load16(d.codes, d.nmask, q_off, qlen, cq = c, qrev, x, nb);
+                            vq = plain_nibbles(nibbles16(x, nb));
+                        }
+                        return vq;
                     };
-                    auto tcode = [&](int p) -> uint32_t {
-                        if ((p >> 4) != ct) { ct = p >> 4; load16(d.codes, d.nmask, t_off, tlen, ct, trev, xt, nt); }
-                        return ((nt >> (p & 15)) & 1u) ? 4u : (xt >> ((p & 15) << 1)) & 3u;
+                    auto tchunk = [&](int c) -> uint64_t {
+                        if (c != ct) {
+                            uint32_t x, nb;
+                            load16(d.codes, d.nmask, t_off, tlen, ct = c, trev, x, nb);
+                            vt = plain_nibbles(nibbles16(x, nb));
+                        }
+                        return vt;
                     };
-                    if (!write_nm_md(d, job, flags, cg, n_ops, qcode, tcode)) st = G3X_ERR_TOO_LONG;
+                    if (!write_nm_md(d, job, flags, cg, n_ops, qchunk, tchunk)) st = G3X_ERR_TOO_LONG;
                 } else if (d.nm) {
                     d.nm[job] = 0;
                     d.md[(int64_t)job * d.md_stride] = 0;

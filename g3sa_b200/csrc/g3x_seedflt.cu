@@ -2,10 +2,11 @@
 // as CHAINFILTERING_flt_chained_seeds_kernel runs it per read, aux.cu:1991-2030) with the window
 // score of mem_seed_sw (aux.cu:117-143).
 //
-// Three steps on the stream: one thread per read turns every seed that mem_seed_sw would align
-// into a g3x_ksw_align2_batch job over the planes (the seed +-50 bases on the read and on the
+// Three steps on the stream: one warp per read turns every seed that mem_seed_sw would align, a lane
+// each, into a g3x_ksw_align2_batch job over the planes (the seed +-50 bases on the read and on the
 // reference, clipped as bns_fetch_seq_gpu clips, bntseq.cu:62-87); one batch aligns them all;
-// one thread per read then keeps, chain by chain and in place, the seeds the reference keeps.
+// one warp per read then keeps, chain by chain and in place, the seeds the reference keeps.  (A thread
+// per read waited for every seed's loads in turn: 107 and 88 us for 1,200 reads of 24 seeds.)
 // mem_seed_sw asks ksw_align2 for start positions (KSW_XSTART) but reads only the score, which
 // the first pass alone decides, so the batch runs without the start-position pass.
 #include <cuda_runtime.h>
@@ -50,19 +51,25 @@ __global__ void sfl_jobs_kernel(g3x_opt_t opt, int32_t min_chain_weight, int64_t
                                 int n_reads, const g3x_chain_t* __restrict__ chains, int n_chains,
                                 const g3x_cseed_t* __restrict__ seeds, int n_seeds, g3x_job_t* __restrict__ jobs,
                                 int32_t* __restrict__ flag, int32_t* __restrict__ min_hsp) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;   // a warp's read
     if (r >= n_reads) return;
     const g3x_read_t rd = reads[r];
-    if (!read_ok(rd, chains, n_chains, n_seeds)) { flag[r] = -1; return; }
+    if (!read_ok(rd, chains, n_chains, n_seeds)) {
+        if (lane == 0) flag[r] = -1;
+        return;
+    }
     const int lq = rd.l_query;
     // float arithmetic where the reference's is float: 1.1f * w, 5.5f * logf(l), 0.05f * l
     const double min_l = min_chain_weight ? (double)(1.1f * (float)min_chain_weight) : (double)(5.5f * logf((float)lq));
-    min_hsp[r] = (int)(opt.a * min_l + .499);
-    if (min_l > (double)(0.05f * (float)lq)) { flag[r] = 0; return; }
-    flag[r] = 1;
+    const bool run = !(min_l > (double)(0.05f * (float)lq));
+    if (lane == 0) {
+        min_hsp[r] = (int)(opt.a * min_l + .499);
+        flag[r] = run;
+    }
+    if (!run) return;
     for (int c = 0; c < rd.n_chains; ++c) {
         const g3x_chain_t ch = chains[rd.chain_beg + c];
-        for (int j = 0; j < ch.n; ++j) {
+        for (int j = lane; j < ch.n; j += 32) {
             const g3x_cseed_t s = seeds[ch.seed_beg + j];
             if (s.len >= kShortLen) continue;                       // aux.cu:124
             int qb = s.qbeg, qe = s.qbeg + s.len;
@@ -101,33 +108,42 @@ __global__ void sfl_keep_kernel(int32_t a, const g3x_read_t* __restrict__ reads,
                                 const g3x_swr_t* __restrict__ sw, const int32_t* __restrict__ sw_status,
                                 const int32_t* __restrict__ flag, const int32_t* __restrict__ min_hsp,
                                 int32_t* __restrict__ sw_score, int32_t* __restrict__ status) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;   // a warp's read
     if (r >= n_reads) return;
     const int fl = flag[r];
-    if (fl < 0) { status[r] = G3X_ERR_INVALID; return; }
+    if (lane == 0) status[r] = fl < 0 ? G3X_ERR_INVALID : G3X_OK;
+    if (fl < 0) return;
+    const int least = min_hsp[r];
     const g3x_read_t rd = reads[r];
     for (int c = 0; c < rd.n_chains; ++c) {
         g3x_chain_t* ch = chains + rd.chain_beg + c;
         const int n = ch->n;
         if (fl == 0) {
             if (sw_score)
-                for (int j = 0; j < n; ++j) sw_score[ch->seed_beg + j] = -2;
+                for (int j = lane; j < n; j += 32) sw_score[ch->seed_beg + j] = -2;
             continue;
         }
         int k = 0;
-        for (int j = 0; j < n; ++j) {
-            const int idx = ch->seed_beg + j;
-            g3x_cseed_t s = seeds[idx];                 // read before slot k <= j is written
-            const int sc = sw_status[idx] == G3X_OK ? sw[idx].score : -1;
-            if (sw_score) sw_score[idx] = sc;
-            if (sc < 0 || sc >= min_hsp[r]) {
+        const int beg = ch->seed_beg;
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const int idx = beg + j0 + lane;
+            g3x_cseed_t s = {};
+            bool keep = false;
+            if (j0 + lane < n) {                        // read before the slots k .. <= j0 + lane are written
+                s = seeds[idx];
+                const int sc = sw_status[idx] == G3X_OK ? sw[idx].score : -1;
+                if (sw_score) sw_score[idx] = sc;
+                keep = sc < 0 || sc >= least;
                 s.score = sc < 0 ? s.len * a : sc;
-                seeds[ch->seed_beg + k++] = s;
             }
+            const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+            if (keep) seeds[beg + k + __popc(kept & ((1u << lane) - 1u))] = s;
+            k += __popc(kept);
+            __syncwarp();                               // (a later chain may hold the same slots)
         }
-        ch->n = k;
+        if (lane == 0) ch->n = k;
+        __syncwarp();
     }
-    status[r] = G3X_OK;
 }
 
 }  // namespace
@@ -168,7 +184,7 @@ extern "C" int g3x_flt_chained_seeds(g3x_ctx* ctx, const g3x_opt_t* opt, int32_t
     int32_t* min_hsp = flag + n_reads;
     const cudaStream_t st = (cudaStream_t)stream;
     if (cudaMemsetAsync(jobs, 0, (size_t)ns * sizeof(g3x_job_t), st) != cudaSuccess) return G3X_ERR_CUDA;
-    const int tb = 128, nb = (n_reads + tb - 1) / tb;
+    const int tb = 128, nb = (n_reads + tb / 32 - 1) / (tb / 32);
     sfl_jobs_kernel<<<nb, tb, 0, st>>>(*opt, min_chain_weight, ref->l_pac, ref->ref_off, ref->d_anns, ref->n_seqs,
                                         d_reads, n_reads, d_chains, n_chains, d_seeds, n_seeds, jobs, flag, min_hsp);
     if (cudaPeekAtLastError() != cudaSuccess) return G3X_ERR_CUDA;

@@ -94,30 +94,58 @@ __device__ __forceinline__ int quad_min(int v) {
     return min(v, __shfl_xor_sync(kFull, v, 2));
 }
 
-// Code of position `pos` of a sequence stored at plane position off (backwards when rev).
-__device__ __forceinline__ uint32_t base_at(const uint32_t* __restrict__ codes, const uint32_t* __restrict__ nmask,
-                                            uint32_t off, int len, int pos, bool rev) {
-    const uint32_t a = off + (uint32_t)(rev ? len - 1 - pos : pos);
-    if ((__ldg(nmask + (a >> 5)) >> (a & 31u)) & 1u) return 4u;
-    return (__ldg(codes + (a >> 4)) >> ((a & 15u) << 1)) & 3u;
+// The quad's query codes, one byte per position: 0-3, 4 for N, 5 from len up to the 8 slen cells of its
+// vectors.  A lane takes every fourth 16-base chunk, so the quad waits for one or two memory
+// latencies (base by base they were a quarter of a 90-base job's time).
+__device__ __forceinline__ void stage_query(const SwDesc& d, uint32_t off, int len, bool rev, int cells, int p,
+                                            uint8_t* qc) {
+    for (int b = 16 * p; b < cells; b += 64) {
+        uint64_t v = 0;
+        if (b < len) {
+            uint32_t x, nb;
+            load16(d.codes, d.nmask, off, len, b >> 4, rev, x, nb);
+            v = nibbles16(x, nb);
+        }
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t h = (uint32_t)(v >> (16 * u)) & 0xFFFFu, t = (h & 0xFFu) | (h & 0xFF00u) << 8;
+            const uint32_t c = (t | t << 4) & 0x0F0F0F0Fu, n = c >> 2 & 0x01010101u;
+            const int valid = len - (b + 4 * u);
+            const uint32_t past = valid >= 4 ? 0u : valid <= 0 ? kFull : kFull << (8 * valid);
+            w[u] = (c & ~(n | n << 1) & ~past) | (0x05050505u & past);
+        }
+        *reinterpret_cast<uint4*>(qc + b) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
 }
 
 // Target rows of a pass: row i is base i of the job's target, or, in the second pass, base
-// te - i for i <= te (the prefix 0..te reversed, ksw.cu:287).  16 bases per refill.
+// te - i for i <= te (the prefix 0..te reversed, ksw.cu:287).  Lane p of the quad holds rows 64 c + 16 p
+// .. + 15 as nibbles (4-7 for N).
 struct Rows {
     uint32_t off, roff;
     int len, rlen, flip;       // flip: rows 0..flip-1 come from the reversed prefix
     bool rev, rrev;
-    int chunk, view;
-    uint32_t x, nb;
-    __device__ __forceinline__ uint32_t code(const uint32_t* codes, const uint32_t* nmask, int i) {
-        const int v = i < flip ? 1 : 0;
-        if (v != view || (i >> 4) != chunk) {
-            view = v; chunk = i >> 4;
-            if (v) load16(codes, nmask, roff, rlen, chunk, rrev, x, nb);
-            else load16(codes, nmask, off, len, chunk, rev, x, nb);
+    uint32_t w0, w1;
+    __device__ __forceinline__ void refill(const uint32_t* codes, const uint32_t* nmask, int i, int p) {
+        const int b = i + 16 * p;
+        uint64_t v = 0;
+        uint32_t x, nb;
+        if (b < flip) {
+            load16(codes, nmask, roff, rlen, b >> 4, rrev, x, nb);
+            v = nibbles16(x, nb);
         }
-        return ((nb >> (i & 15)) & 1u) ? 4u : (x >> ((i & 15) << 1)) & 3u;
+        if (b + 16 > flip && b < len) {
+            load16(codes, nmask, off, len, b >> 4, rev, x, nb);
+            const uint64_t keep = b < flip ? ((uint64_t)1 << (4 * (flip - b))) - 1u : 0u;
+            v = (v & keep) | (nibbles16(x, nb) & ~keep);
+        }
+        w0 = (uint32_t)v;
+        w1 = (uint32_t)(v >> 32);
+    }
+    __device__ __forceinline__ uint32_t code(int i, int lane) const {
+        const uint32_t w = __shfl_sync(kFull, (i & 8) ? w1 : w0, (lane & ~3) | (i >> 4 & 3));
+        return w >> ((i & 7) << 2) & 7u;
     }
 };
 
@@ -183,8 +211,9 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
     for (int i = 0;; ++i) {
         run = run && i < tlen;
         if (!__any_sync(kFull, run)) break;
-        uint2 pool = make_uint2(0u, 0u);
-        if (run) pool = tab[rows.code(d.codes, d.nmask, i)];
+        if ((i & 63) == 0 && run) rows.refill(d.codes, d.nmask, i, p);
+        uint2 pool = tab[rows.code(i, lane)];
+        if (!run) pool = make_uint2(0u, 0u);
         uint32_t hd = shift_up(__viaddmax_s16x2(fc, pc.last, H[MAXSEG - 1]), p);
         uint32_t f = 0u, mx = 0u, dec = d.dec0;
         // the row (ksw.cu:193-208): M = H(i-1, j-1) + S, H = max(M, E, F), E' and F' from H
@@ -251,11 +280,10 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
     }
 }
 
-// One pass of ksw_i16 (ksw.cu:155-262) for the quad's job (live), query codes qcode(pos) for
-// pos < qlen.  With `sub`, row maxima >= minsc go to the job's list (ksw.cu:223-232; lane p = 0
+// One pass of ksw_i16 (ksw.cu:155-262) for the quad's job (live), query codes qc (stage_query).  With `sub`, row maxima >= minsc go to the job's list (ksw.cu:223-232; lane p = 0
 // keeps it) and *nb receives its length.
-template <int MAXSEG, typename QCode>
-__device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen, int tlen, QCode qcode, Rows rows,
+template <int MAXSEG>
+__device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen, int tlen, const uint8_t* qc, Rows rows,
                                            int minsc, int endsc, uint32_t* sub, int* nb, uint32_t* hm,
                                            const uint2* tab, int lane) {
     const int p = lane & 3;
@@ -273,8 +301,8 @@ __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen,
             uint32_t c0 = 5u, c1 = 5u;
             if (live && j >= 0) {
                 const int p0 = j + 2 * p * slen, p1 = p0 + slen;
-                if (p0 < qlen) c0 = qcode(p0);
-                if (p1 < qlen) c1 = qcode(p1);
+                c0 = qc[p0];
+                c1 = qc[p1];
             }
             v |= sel_of(c0, c1) << (16 * u);
         }
@@ -342,10 +370,13 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
     constexpr int QMAX = 8 * MAXSEG;
     __shared__ __align__(16) uint8_t qcodes[kWarps][kQuads][QMAX];
     __shared__ uint32_t snap[kWarps][MAXSEG * 32];
-    __shared__ uint2 tab[5];
+    __shared__ uint2 tab[8];
     pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane >> 2, p = lane & 3;
-    if (threadIdx.x < 5) tab[threadIdx.x] = make_uint2(d.tab[2 * threadIdx.x], d.tab[2 * threadIdx.x + 1]);
+    if (threadIdx.x < 8) {
+        const int a = threadIdx.x < 4 ? threadIdx.x : 4;
+        tab[threadIdx.x] = make_uint2(d.tab[2 * a], d.tab[2 * a + 1]);
+    }
     __syncthreads();
     uint8_t* qc = qcodes[warp][quad];
     uint32_t* hm = snap[warp];
@@ -383,14 +414,13 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
         Rows rows;
         rows.off = live ? jb.t_off : 0u; rows.len = tlen; rows.rev = trev;
         rows.roff = 0u; rows.rlen = 0; rows.rrev = false; rows.flip = 0;
-        rows.chunk = -1; rows.view = -1; rows.x = 0u; rows.nb = 0u;
+        rows.w0 = rows.w1 = 0u;
         if constexpr (!SECOND) {
-            if (live)
-                for (int pos = p; pos < qlen; pos += 4) qc[pos] = (uint8_t)base_at(d.codes, d.nmask, jb.q_off, qlen, pos, qrev);
+            if (live) stage_query(d, jb.q_off, qlen, qrev, (qlen + 7) & ~7, p, qc);
             __syncwarp();
             uint32_t* sub = subo && live ? d.sub + (int64_t)job * d.sub_stride : nullptr;
             int n_b = 0;
-            const PassOut r = sw_pass<MAXSEG>(d, live, qlen, tlen, [&](int pos) { return (uint32_t)qc[pos]; }, rows,
+            const PassOut r = sw_pass<MAXSEG>(d, live, qlen, tlen, qc, rows,
                                               minsc, endsc, sub, &n_b, hm, tab, lane);
             g3x_swr_t o{r.score, r.te, r.qe, -1, -1, -1, -1};
             // second best: list entries more than ceil(score / max(mat)) rows from te (ksw.cu:249-256)
@@ -410,14 +440,14 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
             int score = 0, te = -1, qe = 0;
             if (live) { score = d.out[job].score; te = d.out[job].te; qe = d.out[job].qe; }
             const int lq = live ? qe + 1 : 0, lt = te + 1;
-            if (live)
-                for (int pos = p; pos < lq; pos += 4) qc[pos] = (uint8_t)base_at(d.codes, d.nmask, jb.q_off, qlen, qe - pos, qrev);
+            // the query's prefix 0..qe backwards
+            if (live) stage_query(d, qrev ? jb.q_off + (uint32_t)(qlen - lq) : jb.q_off, lq, !qrev, (lq + 7) & ~7, p, qc);
             __syncwarp();
             rows.flip = lt;
             rows.rlen = lt;
             if (!trev) { rows.roff = rows.off; rows.rrev = true; }
             else { rows.roff = rows.off + (uint32_t)(tlen - lt); rows.rrev = false; }
-            const PassOut rr = sw_pass<MAXSEG>(d, live, lq, tlen, [&](int pos) { return (uint32_t)qc[pos]; }, rows,
+            const PassOut rr = sw_pass<MAXSEG>(d, live, lq, tlen, qc, rows,
                                                kNoScore, score, nullptr, nullptr, hm, tab, lane);
             if (live && p == 0 && rr.score == score) {      // kept when it finds the same score
                 d.out[job].tb = te - rr.te;
