@@ -24,12 +24,13 @@
 // cell never wraps.  Longer queries get G3X_ERR_TOO_LONG.
 //
 // Jobs are sorted by segment count and rows (a device counting sort), so a warp's eight jobs have
-// the same segments and about the same rows; each of three launches (8, 16, 32 segments) takes
-// its class's range from a device counter.  The second pass for the start positions (KSW_XSTART) has
+// the same segments and about the same rows; each of three launches (registers for 8, 16, 32
+// segments) takes its classes of four segment counts from device counters.  The second pass for the start positions (KSW_XSTART) has
 // its own sort and launches.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include <type_traits>
 #include "g3x_core.h"
 #include "g3x_internal.h"
 #include "g3x_stage.cuh"
@@ -42,6 +43,7 @@ constexpr int kQuads = 8;                 // jobs per warp
 constexpr int kWarps = 4;                 // warps per block
 constexpr int kRowBins = 128;             // rows, eight bins per doubling
 constexpr int kSegBins = 32;              // segments 1..32
+constexpr int kClasses = kSegBins / 4;    // 29-32 segments first
 constexpr int kBins = kSegBins * kRowBins + 1;   // + the bin of rejected jobs (qlen 0 or > 256)
 constexpr int kNoScore = 0x10000;         // minsc / endsc when the flag is absent (ksw.cu:176-177)
 
@@ -50,8 +52,8 @@ struct SwDesc {
     const uint32_t* codes;
     const uint32_t* nmask;
     const int32_t* order;      // job indices, sorted
-    const int32_t* range;      // [offset, count] of this launch's jobs in `order`
-    int32_t* queue;            // this launch's slot counter (zeroed)
+    const int32_t* range;      // [offset, count] in `order` of each class of four segment counts
+    int32_t* queue;            // the classes' slot counters (zeroed)
     g3x_swr_t* out;
     int32_t* status;
     uint32_t* sub;             // XSUBO: row maxima per job (imax << 16 | row), sub_stride each
@@ -168,11 +170,6 @@ struct PassOut {
     int score, te, qe;
 };
 
-// Slot cases 0..31 of the unrolled segment loops.  A loop enters at the warp's first used slot
-// with one jump (a switch on a warp-uniform value) and falls through the rest.
-#define G3X_SW_CASES(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) \
-    F(15) F(16) F(17) F(18) F(19) F(20) F(21) F(22) F(23) F(24) F(25) F(26) F(27) F(28) F(29) F(30) F(31)
-
 // Constants of a pass: the score steps of SwDesc as int16x2 and what a job's segment count makes of
 // the insertion extension.
 struct PassConst {
@@ -180,10 +177,47 @@ struct PassConst {
     uint32_t d1, d2, d4;       // decay of F over 1, 2 and 4 cells of the vector (slen segments each)
 };
 
-// The row loop of one pass over registers H, E (slot MAXSEG - slen + j = segment j).  UNI: every
-// live quad of the warp has the same slot base, so no slot needs a per-quad guard; a quad that
-// is not running computes on slots it never reads back.  SYM: equal insertion and deletion costs,
-// so E and F share H - (o + e).  WIDE: see below.
+// The segments of a row, slots S .. MAXSEG - 1 (S0: the row's first).
+template <int MAXSEG, int S0, bool SYM, bool WIDE, int S = S0>
+__device__ __forceinline__ void seg_steps(const SwDesc& d, const uint2 pool, const uint32_t (&sel)[sel_words(MAXSEG)],
+                                          int base, uint32_t (&H)[MAXSEG], uint32_t (&E)[MAXSEG], uint32_t& hd,
+                                          uint32_t& f, uint32_t& mx, uint32_t& dec, uint32_t& fc) {
+    if constexpr (S < MAXSEG) {
+        const bool mine = S >= S0 + 3 || S >= base;      // (known for all but three slots)
+        const uint32_t sc = prmt(pool.x, pool.y, sel_at<MAXSEG, S>(sel));
+        uint32_t h = __viaddmax_s16x2(hd, sc, __vimax_s16x2_relu(E[S], f));
+        uint32_t raised, fc2 = fc, dec2 = dec;
+        if constexpr (WIDE) {
+            raised = __vimax_s16x2_relu(H[S], fc);
+            fc2 = __viaddmax_s16x2_relu(fc, d.nstep, 0u);
+        } else {
+            raised = __viaddmax_s16x2(fc, dec, H[S]);
+            dec2 = dec * d.one + d.step;
+        }
+        if constexpr (S < S0 + 3) {
+            h = mine ? h : 0u;
+            raised = mine ? raised : hd;
+            fc2 = mine ? fc2 : fc;
+            dec2 = mine ? dec2 : dec;
+        }
+        hd = raised; fc = fc2; dec = dec2;
+        // two segments at a time
+        if constexpr (S & 1) mx = __vimax3_s16x2(mx, H[S - 1], h);
+        H[S] = h;
+        const uint32_t td = __viaddmax_s16x2_relu(h, d.noedel, 0u);
+        E[S] = __viaddmax_s16x2(E[S], d.nedel, td);
+        f = __viaddmax_s16x2(f, d.neins, SYM ? td : __viaddmax_s16x2_relu(h, d.noeins, 0u));
+        seg_steps<MAXSEG, S0, SYM, WIDE, S + 1>(d, pool, sel, base, H, E, hd, f, mx, dec, fc);
+    }
+}
+
+// The row loop of one pass over registers H, E (slot MAXSEG - slen + j = segment j), over the last V
+// slots: every live quad of the warp has V - 3 .. V segments, so only the first four slots ask
+// whether they are the quad's (a slot before its first segment holds zeros: score 0, no H, E or F),
+// and the others are straight code.  (One jump per row to a first slot common to the warp, and a guard
+// in every slot where there was none, took 390 instructions a row of 12 segments.)  A quad that is
+// not running computes on slots it never reads back.  SYM: equal insertion and deletion costs, so
+// E and F share H - (o + e).  WIDE: see below.
 //
 // The lazy-F loop (ksw.cu:209-220) in closed form.  It moves F up one cell, folds it into H segment
 // by segment as it decays, E untouched, round after round, until no cell's F - e beats its
@@ -199,11 +233,12 @@ struct PassConst {
 // C + e) is one 32-bit addition a segment on both halves, exact while it fits 16 bits.  WIDE: gap
 // extensions above 1000 decay C by a saturating step instead; so does o = 0, where the loop stops
 // after the first segment of the first round and raises nothing else.
-template <int MAXSEG, bool UNI, bool SYM, bool WIDE>
+template <int MAXSEG, int V, bool SYM, bool WIDE>
 __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Rows& rows, int minsc, int endsc,
                                         uint32_t* sub, int& n_b, uint32_t (&H)[MAXSEG], uint32_t (&E)[MAXSEG],
                                         const uint32_t (&sel)[sel_words(MAXSEG)], const PassConst& pc, int base,
-                                        int base_min, uint32_t* hm, const uint2* tab, int lane, int& gmax, int& te) {
+                                        uint32_t* hm, const uint2* tab, int lane, int& gmax, int& te) {
+    constexpr int S0 = MAXSEG - V;
     const int p = lane & 3;
     int last_row = -2, last_v = 0;
     bool run = live;
@@ -217,32 +252,7 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
         uint32_t hd = shift_up(__viaddmax_s16x2(fc, pc.last, H[MAXSEG - 1]), p);
         uint32_t f = 0u, mx = 0u, dec = d.dec0;
         // the row (ksw.cu:193-208): M = H(i-1, j-1) + S, H = max(M, E, F), E' and F' from H
-        switch (base_min) {
-#define G3X_SW_MAIN(S)                                                                               \
-    case S:                                                                                          \
-        if constexpr (S < MAXSEG) {                                                                  \
-            if (UNI || S >= base) {                                                                  \
-                const uint32_t sc = prmt(pool.x, pool.y, sel_at<MAXSEG, S>(sel));                    \
-                const uint32_t h = __viaddmax_s16x2(hd, sc, __vimax_s16x2_relu(E[S], f));            \
-                if constexpr (WIDE) {                                                                \
-                    hd = __vimax_s16x2_relu(H[S], fc);                                               \
-                    fc = __viaddmax_s16x2_relu(fc, d.nstep, 0u);                                     \
-                } else {                                                                             \
-                    hd = __viaddmax_s16x2(fc, dec, H[S]);                                            \
-                    dec = dec * d.one + d.step;                                                      \
-                }                                                                                    \
-                H[S] = h;                                                                            \
-                /* two segments at a time (a slot before the job's first holds zeros) */            \
-                if constexpr (S & 1) mx = __vimax3_s16x2(mx, H[S - 1], h);                           \
-                const uint32_t td = __viaddmax_s16x2_relu(h, d.noedel, 0u);                          \
-                E[S] = __viaddmax_s16x2(E[S], d.nedel, td);                                          \
-                f = __viaddmax_s16x2(f, d.neins, SYM ? td : __viaddmax_s16x2_relu(h, d.noeins, 0u)); \
-            }                                                                                        \
-        }
-            G3X_SW_CASES(G3X_SW_MAIN)
-#undef G3X_SW_MAIN
-            default: break;
-        }
+        seg_steps<MAXSEG, S0, SYM, WIDE>(d, pool, sel, base, H, E, hd, f, mx, dec, fc);
         // the F carried into each cell (a lane a shuffle leaves alone meets its own, decayed)
         f = shift_up(f, p);
         f = __viaddmax_s16x2(shift_up(f, p), pc.d1, f);
@@ -264,16 +274,8 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
             }
             if (im > gmax) {                        // ksw.cu:233-238
                 gmax = im; te = i;
-                switch (base_min) {
-#define G3X_SW_SNAP(S)                                                                               \
-    case S:                                                                                          \
-        if constexpr (S < MAXSEG) {                                                                  \
-            if (UNI || S >= base) hm[S * 32 + lane] = H[S];                                          \
-        }
-                    G3X_SW_CASES(G3X_SW_SNAP)
-#undef G3X_SW_SNAP
-                    default: break;
-                }
+#pragma unroll
+                for (int S = S0; S < MAXSEG; ++S) hm[S * 32 + lane] = H[S];
                 if (gmax >= endsc) run = false;
             }
         }
@@ -282,15 +284,13 @@ __device__ __forceinline__ void sw_rows(const SwDesc& d, bool live, int tlen, Ro
 
 // One pass of ksw_i16 (ksw.cu:155-262) for the quad's job (live), query codes qc (stage_query).  With `sub`, row maxima >= minsc go to the job's list (ksw.cu:223-232; lane p = 0
 // keeps it) and *nb receives its length.
-template <int MAXSEG>
+template <int MAXSEG, int V>
 __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen, int tlen, const uint8_t* qc, Rows rows,
                                            int minsc, int endsc, uint32_t* sub, int* nb, uint32_t* hm,
                                            const uint2* tab, int lane) {
     const int p = lane & 3;
     const int slen = live ? (qlen + 7) >> 3 : 0;
     const int base = MAXSEG - slen;
-    const int base_min = (int)__reduce_min_sync(kFull, (unsigned)base);
-    const bool uni = __all_sync(kFull, !live || base == base_min);
     uint32_t H[MAXSEG], E[MAXSEG], sel[sel_words(MAXSEG)];
 #pragma unroll
     for (int s = 0; s < MAXSEG; s += 2) {
@@ -319,18 +319,12 @@ __device__ __forceinline__ PassOut sw_pass(const SwDesc& d, bool live, int qlen,
     const int64_t seg = (int64_t)slen * d.carry_e;
     const bool wide = d.one == 0u;
     const PassConst pc{neg_pair(wide ? seg - d.carry_e : seg), neg_pair(seg), neg_pair(2 * seg), neg_pair(4 * seg)};
-#define G3X_SW_ROWS(UNI, SYM, WIDE)                                                                              \
-    sw_rows<MAXSEG, UNI, SYM, WIDE>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel, pc, base, base_min, hm, \
-                                    tab, lane, gmax, te)
-    if (wide) {
-        G3X_SW_ROWS(false, false, true);
-    } else if (d.noedel == d.noeins) {
-        if (uni) G3X_SW_ROWS(true, true, false);
-        else G3X_SW_ROWS(false, true, false);
-    } else {
-        if (uni) G3X_SW_ROWS(true, false, false);
-        else G3X_SW_ROWS(false, false, false);
-    }
+#define G3X_SW_ROWS(SYM, WIDE)                                                                                    \
+    sw_rows<MAXSEG, V, SYM, WIDE>(d, live, tlen, rows, minsc, endsc, sub, n_b, H, E, sel, pc, base, hm, tab, lane, gmax, te)
+    // SYM: equal insertion and deletion costs, so E and F share H - (o + e)
+    if (wide) G3X_SW_ROWS(false, true);
+    else if (d.noedel == d.noeins) G3X_SW_ROWS(true, false);
+    else G3X_SW_ROWS(false, false);
 #undef G3X_SW_ROWS
     __syncwarp();
     // end on the query: the smallest position holding the best row's largest cell, cells read
@@ -380,13 +374,16 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
     __syncthreads();
     uint8_t* qc = qcodes[warp][quad];
     uint32_t* hm = snap[warp];
-    const int off = d.range[0], cnt = d.range[1];
     const bool subo = (d.xtra & G3X_KSW_XSUBO) != 0;
     const int minsc = subo ? d.xtra & 0xFFFF : kNoScore;
     const int endsc = (d.xtra & G3X_KSW_XSTOP) ? d.xtra & 0xFFFF : kNoScore;
+    // the jobs of V - 3 .. V segments, class k of the sort
+    auto run_class = [&](auto v, int k) {
+    constexpr int V = decltype(v)::value;
+    const int off = d.range[2 * k], cnt = d.range[2 * k + 1];
     for (;;) {
         int first = 0;
-        if (lane == 0) first = atomicAdd(d.queue, kQuads);
+        if (lane == 0) first = atomicAdd(d.queue + k, kQuads);
         first = __shfl_sync(kFull, first, 0);
         if (first >= cnt) break;
         const int slot = first + quad;
@@ -420,7 +417,7 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
             __syncwarp();
             uint32_t* sub = subo && live ? d.sub + (int64_t)job * d.sub_stride : nullptr;
             int n_b = 0;
-            const PassOut r = sw_pass<MAXSEG>(d, live, qlen, tlen, qc, rows,
+            const PassOut r = sw_pass<MAXSEG, V>(d, live, qlen, tlen, qc, rows,
                                               minsc, endsc, sub, &n_b, hm, tab, lane);
             g3x_swr_t o{r.score, r.te, r.qe, -1, -1, -1, -1};
             // second best: list entries more than ceil(score / max(mat)) rows from te (ksw.cu:249-256)
@@ -447,7 +444,7 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
             rows.rlen = lt;
             if (!trev) { rows.roff = rows.off; rows.rrev = true; }
             else { rows.roff = rows.off + (uint32_t)(tlen - lt); rows.rrev = false; }
-            const PassOut rr = sw_pass<MAXSEG>(d, live, lq, tlen, qc, rows,
+            const PassOut rr = sw_pass<MAXSEG, V>(d, live, lq, tlen, qc, rows,
                                                kNoScore, score, nullptr, nullptr, hm, tab, lane);
             if (live && p == 0 && rr.score == score) {      // kept when it finds the same score
                 d.out[job].tb = te - rr.te;
@@ -456,6 +453,18 @@ __global__ void __launch_bounds__(128, MAXSEG == 32 ? 4 : MAXSEG == 16 ? 6 : 8) 
         }
         __syncwarp();
     }
+    };
+#define G3X_SW_CLASS(V) run_class(std::integral_constant<int, (V)>(), (kSegBins - (V)) / 4)
+    if constexpr (MAXSEG == 32) {
+        G3X_SW_CLASS(32);
+        G3X_SW_CLASS(28);
+        G3X_SW_CLASS(24);
+        G3X_SW_CLASS(20);
+    } else {
+        G3X_SW_CLASS(MAXSEG);
+        G3X_SW_CLASS(MAXSEG - 4);
+    }
+#undef G3X_SW_CLASS
     pdl_chain_end();
 }
 
@@ -485,8 +494,8 @@ __global__ void sw_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, const g
     if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(hist + b, __popc(peers));
 }
 
-// Exclusive scan of the bins (one block) and the three launches' ranges: 17-32 segments, 9-16,
-// and 1-8, in the first pass together with the rejected bin (with_last).
+// Exclusive scan of the bins (one block) and the classes' ranges, the last (1-4 segments) in the
+// first pass together with the rejected bin (with_last).
 __global__ void __launch_bounds__(1024) sw_scan_kernel(const int32_t* __restrict__ hist, int32_t* __restrict__ cursor,
                                                        int32_t* __restrict__ range, int with_last) {
     constexpr int kPer = (kBins + 1023) / 1024;
@@ -513,12 +522,11 @@ __global__ void __launch_bounds__(1024) sw_scan_kernel(const int32_t* __restrict
         at += v[u];
     }
     __syncthreads();
-    if (t == 0) {
-        const int c16 = cursor[(kSegBins - 16) * kRowBins], c8 = cursor[(kSegBins - 8) * kRowBins];
-        const int last = cursor[kBins - 1] + (with_last ? hist[kBins - 1] : 0);
-        range[0] = 0;   range[1] = c16;
-        range[2] = c16; range[3] = c8 - c16;
-        range[4] = c8;  range[5] = last - c8;
+    if (t < kClasses) {
+        const int lo = cursor[4 * t * kRowBins];
+        const int hi = cursor[4 * (t + 1) * kRowBins] + (t == kClasses - 1 && with_last ? hist[kBins - 1] : 0);
+        range[2 * t] = lo;
+        range[2 * t + 1] = hi - lo;
     }
 }
 
@@ -538,10 +546,7 @@ __global__ void sw_scatter_kernel(const int32_t* __restrict__ bin, int n, int32_
 uint32_t pack16(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; }
 
 template <int MAXSEG, bool SECOND>
-int launch_class(const SwDesc& d0, const int32_t* range, int32_t* queue, bool first, cudaStream_t st) {
-    SwDesc d = d0;
-    d.range = range;
-    d.queue = queue;
+int launch_classes(const SwDesc& d, bool first, cudaStream_t st) {
     auto kern = sw_kernel<MAXSEG, SECOND>;
     const int per_sm = resident_blocks(kern, 32 * kWarps, 0);
     // the classes of a pass run side by side: programmatic dependents of one another
@@ -559,15 +564,17 @@ int launch_class(const SwDesc& d0, const int32_t* range, int32_t* queue, bool fi
 
 // One pass over the jobs: sorted, then a launch per class.
 template <bool SECOND>
-int run_pass(const SwDesc& d, int32_t n, int32_t* buf, cudaStream_t st) {
+int run_pass(const SwDesc& d0, int32_t n, int32_t* buf, cudaStream_t st) {
     int32_t* bin = buf;
     int32_t* order = bin + n;
     int32_t* hist = order + n;
     int32_t* cursor = hist + kBins;
-    int32_t* range = cursor + kBins;      // 6 used, 8 kept
-    int32_t* queue = range + 8;           // 3 used, 4 kept
+    int32_t* range = cursor + kBins;
+    int32_t* queue = range + 2 * kClasses;
+    SwDesc d = d0;
+    d.order = order; d.range = range; d.queue = queue;
     if (cudaMemsetAsync(hist, 0, sizeof(int32_t) * kBins, st) != cudaSuccess ||
-        cudaMemsetAsync(queue, 0, sizeof(int32_t) * 4, st) != cudaSuccess)
+        cudaMemsetAsync(queue, 0, sizeof(int32_t) * kClasses, st) != cudaSuccess)
         return G3X_ERR_CUDA;
     const int min_score = (d.xtra & G3X_KSW_XSUBO) ? d.xtra & 0xFFFF : -1;
     const int tb = 256, nb = (n + tb - 1) / tb;
@@ -576,9 +583,9 @@ int run_pass(const SwDesc& d, int32_t n, int32_t* buf, cudaStream_t st) {
     sw_scatter_kernel<<<nb, tb, 0, st>>>(bin, n, cursor, order);
     if (cudaPeekAtLastError() != cudaSuccess) return G3X_ERR_CUDA;
     int rc;
-    if ((rc = launch_class<32, SECOND>(d, range, queue, true, st))) return rc;
-    if ((rc = launch_class<16, SECOND>(d, range + 2, queue + 1, false, st))) return rc;
-    return launch_class<8, SECOND>(d, range + 4, queue + 2, false, st);
+    if ((rc = launch_classes<32, SECOND>(d, true, st))) return rc;
+    if ((rc = launch_classes<16, SECOND>(d, false, st))) return rc;
+    return launch_classes<8, SECOND>(d, false, st);
 }
 
 }  // namespace
@@ -604,7 +611,7 @@ extern "C" int g3x_ksw_align2_batch(g3x_ctx* ctx, const g3x_score_t* score, cons
     const int dev = ctx_device(ctx);
     if (cudaSetDevice(dev) != cudaSuccess) return G3X_ERR_CUDA;
     SwScratch& s = ctx_sw(ctx);
-    const int64_t need = (int64_t)2 * n + 2 * kBins + 8 + 4;
+    const int64_t need = (int64_t)2 * n + 2 * kBins + 3 * kClasses;
     const int64_t sub_need = subo ? (int64_t)n * std::max(max_tlen, 1) : 0;
     if (s.cap < need || s.sub_cap < sub_need) {
         const int64_t cap = std::max(need, s.cap), sub_cap = std::max(sub_need, s.sub_cap);
@@ -620,7 +627,7 @@ extern "C" int g3x_ksw_align2_batch(g3x_ctx* ctx, const g3x_score_t* score, cons
     const cudaStream_t st = (cudaStream_t)stream;
     SwDesc d;
     memset(&d, 0, sizeof(d));
-    d.jobs = d_jobs; d.codes = d_codes; d.nmask = d_nmask; d.order = s.buf + n;
+    d.jobs = d_jobs; d.codes = d_codes; d.nmask = d_nmask;
     d.out = d_out; d.status = d_status;
     d.sub = subo ? s.sub : nullptr;
     d.sub_stride = subo ? std::max(max_tlen, 1) : 0;
