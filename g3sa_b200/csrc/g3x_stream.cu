@@ -257,8 +257,6 @@ int extend_seeds_stream(StreamScratch& ss, const g3x_opt_t& opt, const ScorePara
             }
         }
         if (!done) {
-            // the last, partial chunk: beside it run the other chunks of its round
-            if (runner) cw[l].at_once = (int32_t)((nchunks - 1) % kStreamLanes + 1);
             LaunchDesc cp = proto;             // the chunk's planes: its copied words, re-based
             cp.n_bases = std::min<int64_t>(cwn * 16, mwn * 32);
             if ((rc = extend_seeds(s.seeds, opt, sp, s.d_seeds, (int)R.count, s.d_codes, s.d_nmask, s.d_regs,
