@@ -24,7 +24,7 @@
 // multiply-adds (the bias keeps both halves non-negative, so one 32-bit subtraction serves both)
 // and clipped to 0 or 1.  A
 // lane's eight cells make one word, a warp's row one 128-byte line of scratch.  The backtrack
-// (ksw.cu:783-806) stays on one index while it moves diagonally, so the group reads G rows of that
+// (ksw.cu:783-806) stays on one index while it moves diagonally, so the group reads 32 rows of that
 // index at a time and takes the run of matches up to the first gap from a ballot; gaps go cell by
 // cell.
 #include <cuda_runtime.h>
@@ -56,7 +56,7 @@ template <int G, bool kSym>
 __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams& sp, const PairConst& pc,
                                           const uint4* from, const uint2* pools, const int32_t* order, int n,
                                           int32_t* queue, uint32_t* z, int lane) {
-    constexpr int kGroups = 32 / G;
+    constexpr int kGroups = 32 / G, K = 32 / G;     // K: rows a lane looks up at a time in the backtrack
     const int r = lane & (G - 1), gb = lane & ~(G - 1);
     const unsigned gmask = (G == 32 ? kAll : ((1u << G) - 1u)) << gb;
     const uint32_t minus = 0u - sp.k16 / 65536u;      // run-time -1: subtract on the multiply-add pipe
@@ -225,16 +225,29 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
             const bool go = inside && i >= 0 && k >= 0 && !full && !bad;
             const int dk = k - i + w;                             // index, the same along a diagonal
             if (go && (dk < 0 || dk > 2 * w)) bad = true;         // never on a path with a finite score
-            const int cells = min(min(i, k) + 1, which ? 1 : G);  // a gap goes on cell by cell
-            uint32_t nib = 0u;
-            if (go && !bad && r < cells) nib = (z[(int64_t)(i - r) * 32 + gb + (dk >> 3)] >> ((dk & 7) << 2)) & 0xFu;
-            // the operation at the cell: from H (M, else E, else F), or the gap going on or not
-            const int o = which == 0 ? ((nib & 1u) ? 1 + (int)(nib >> 1 & 1u) : 0) : (nib >> (which + 1)) & 1u ? which : 0;
-            const unsigned gap = __ballot_sync(kAll, go && r < cells && o != 0) & gmask;
+            const int cells = min(min(i, k) + 1, which ? 1 : 32); // a gap goes on cell by cell
+            // lane r: rows i - K r .. i - K r - (K - 1); its first cell that is no match, and the
+            // operation there: from H (M, else E, else F), or the gap going on or not
+            uint32_t dirs[K];
+#pragma unroll
+            for (int t = 0; t < K; ++t) {
+                dirs[t] = 0u;
+                if (go && !bad && K * r + t < cells) dirs[t] = z[(int64_t)(i - K * r - t) * 32 + gb + (dk >> 3)];
+            }
+            int stop_at = K, o = 0;
+#pragma unroll
+            for (int t = K - 1; t >= 0; --t) {
+                const uint32_t nib = dirs[t] >> ((dk & 7) << 2);
+                const int ot = which == 0 ? ((nib & 1u) ? 1 + (int)(nib >> 1 & 1u) : 0) : (nib >> (which + 1)) & 1u ? which : 0;
+                o = ot ? ot : o;
+                stop_at = ot ? t : stop_at;
+            }
+            const unsigned gap = __ballot_sync(kAll, stop_at < K) & gmask;
             const int at = gap ? __ffs(gap) - 1 : 0;
             const int og = __shfl_sync(kAll, o, at);
+            const int before = __shfl_sync(kAll, stop_at, at) + K * (at - gb);
             if (go && !bad) {
-                const int run = gap ? at - gb : cells;
+                const int run = gap ? before : cells;
                 if (run) { push(0, run); i -= run; k -= run; which = 0; }
                 if (gap && !full) {
                     if (og == 1) { push(2, 1); --i; } else { push(1, 1); --k; }
@@ -289,7 +302,7 @@ __device__ __forceinline__ void run_pairs(const GlobalDesc& d, const ScoreParams
 // d.range null: the jobs as they are numbered, a warp each.  Else [offset, count] of the classes
 // of d.order, class k in groups of 2 << k lanes, the widest first.
 template <bool kSym>
-__global__ void __launch_bounds__(32 * kGlobal16Warps) global16_kernel(GlobalDesc d, ScoreParams sp) {
+__global__ void __launch_bounds__(32 * kGlobal16Warps, 11) global16_kernel(GlobalDesc d, ScoreParams sp) {
     __shared__ uint4 from[9];          // pair words of the columns at or right of an offset
     __shared__ uint2 pools[8];
     if (threadIdx.x < 9) {
