@@ -193,7 +193,7 @@ static ClassRes ctx_res(g3x_ctx* ctx) {
 // settings).  Queries beyond the lane classes run in the band kernel where a window holds their
 // band: 1,500 segments of 500-5,000 bases at w = 500 take 32.8 ms row-parallel, which sweeps the row in
 // shared memory tile by tile, and 7.5 ms with the band's row in registers; 20,000 at w = 100 162 and
-// 21.  Shorter ones are here only for their scores, a few jobs not worth three launches.  queue:
+// 8.1.  Shorter ones are here only for their scores, a few jobs not worth three launches.  queue:
 // four zeroed counters.
 static int launch_last(const LaunchDesc& d, const ScoreParams& sp, int32_t* queue, cudaStream_t st) {
     LaunchDesc r = d;
@@ -283,31 +283,31 @@ static int launch_classes(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParam
 }
 
 // The group-per-job kernel or the width classes.  A lane class lasts as long as its longest job
-// (0.5-1.1 ms at 250 bases, whatever its job count) and then costs 5.5-8 ns a job; a group costs
-// 17-23 ns a job and 0.1 ms at least.  Measured on batches of uneven left and right extensions, group
-// against lanes: 62 jobs 113 and 606 us, 9.9k jobs 290 and 1107, 19.8k 403 and 1041, 39.6k 709 and
-// 1148, 79k 1343 and 1108; right extensions of 1-150 bases: 20k 504 and 960, 40k 925 and 973; w = 30:
-// 19.8k 344 and 541, 39.6k 592 and 579.  So batches up to 32k jobs take the groups.  A seed call
-// (left wave, right wave and their retry waves) pays the lanes' latency more often: 20k seeds 904 and
-// 2319 us, 40k 1520 and 2379, 80k 2814 and 2360, so its waves take them up to 48k.  Waves that run
-// side by side (the seed stream's) fill the lanes together and count together.
-constexpr int64_t kGroupJobs = 32768, kGroupSeeds = 49152;
+// (0.5-1.1 ms at 250 bases, whatever its job count) and then costs 5.2-8 ns a job; a group costs
+// 14-22 ns a job and 0.1 ms at least.  Measured on batches of uneven left and right extensions, group
+// against lanes: 62 jobs 113 and 606 us, 9.9k jobs 259 and 1063, 19.8k 376 and 1065, 39.6k 634 and
+// 1079, 79k 1155 and 1115; right extensions of 1-150 bases: 20k 449 and 892, 40k 809 and 926, 60k 1177
+// and 946; w = 30: 39.6k 537 and 554, 59k 745 and 558.  So batches up to 36k jobs take the groups; from
+// there on narrow bands gain nothing, and the order a caller chose (by length or learned), which the
+// groups ignore, keeps deciding.  A seed call (left wave, right wave and their retry waves) pays the
+// lanes' latency more often: 20k seeds 846 and 2171 us, 40k 1360 and 2310, 60k 1884 and 2356, so its
+// waves take them up to 72k.  Waves that run side by side (the seed stream's) fill the lanes together
+// and count together.
+constexpr int64_t kGroupJobs = 36864, kGroupSeeds = 73728;
 // Up to here a job takes a warp in the order given: 62 jobs 113 us against 126 sorted into classes
-// (three launches less), 2k 190 against 216, 4k 249 against 264 and, for the shorter right
-// extensions, 5k 295 against 248.
-constexpr int64_t kDirectJobs = 3072;
+// (three launches less), 2k 186 against 205, 4k 227 against 240, 6k 273 against 252; seed calls of
+// 3k 449 against 566, 5k 543 against 577, 10k 813 against 601.
+constexpr int64_t kDirectJobs = 4096, kDirectSeeds = 5120;
 
 // Contexts with width classes of their own (g3x_set_tiles), in int32 or with class timing keep to
 // them.
 static bool groups_allowed(const g3x_ctx* ctx) { return !ctx->tiles_set && !ctx->no_int16 && !ctx->timing; }
 
 // Runs a batch (or with base.order a wave of at most base.n jobs) through the group-per-job
-// kernel: up to kDirectJobs jobs as they are listed, a warp each; beyond, sorted into the
-// kernel's classes, up to eight jobs a warp.  The jobs it cannot take follow in the row-parallel
-// kernel.
-static int run_grouped(const LaunchDesc& base, const ScoreParams& sp, SchedScratch& s, int32_t* queue,
+// kernel: as they are listed, a warp each (direct), or sorted into the kernel's classes, up to eight
+// jobs a warp.  The jobs it cannot take follow as the last class's.
+static int run_grouped(const LaunchDesc& base, const ScoreParams& sp, SchedScratch& s, int32_t* queue, bool direct,
                        cudaStream_t st) {
-    const bool direct = base.n <= kDirectJobs;
     LaunchDesc rest = base;
     int rc;
     if (cudaMemsetAsync(queue, 0, kQueueInts * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
@@ -347,7 +347,7 @@ static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams
         LaunchDesc d = base;
         d.stats = ctx->d_stats;
         if (cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), st) != cudaSuccess) return G3X_ERR_CUDA;
-        return run_grouped(d, sp, ctx->sched, ctx->d_queue, st);
+        return run_grouped(d, sp, ctx->sched, ctx->d_queue, base.n <= kDirectJobs, st);
     }
     rc = learned && ctx->model.active
              ? schedule_jobs_learned(ctx->sched, base.jobs, base.n, base.codes, base.nmask, base.n_bases,
@@ -368,7 +368,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     // A retry wave holds the few jobs whose band was too narrow (their count stays on the device):
     // in groups it lasts 0.1 ms where a lane class of a handful of jobs lasts 0.5.
     if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= kGroupSeeds))
-        return run_grouped(d, sp, sched, res.queue, st);
+        return run_grouped(d, sp, sched, res.queue, d.n <= kDirectSeeds, st);
     int rc = w->learned && ctx->model.active
                  ? schedule_jobs_learned(sched, d.jobs, d.n, d.codes, d.nmask, d.n_bases, ctx->model.params, sp,
                                          ctx->tiles, st, d.order, d.count)

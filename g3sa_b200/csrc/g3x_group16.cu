@@ -4,23 +4,23 @@
 // The lane-per-job kernel (g3x_lane16.cu) needs tens of thousands of jobs: a lane walks its row
 // block by block, 2,000-3,400 cycles a row for 200 columns, so a batch lasts as long as its
 // longest job (0.5-0.6 ms at 250 bases) however few jobs it has.  Here a group of G lanes runs a
-// job and a row is one step: lane r of the group holds columns 8r .. 8r + 7 of the row buffer
-// (ksw.cu:310) in registers for the whole job, as the same four int16x2 words of H and four of E
-// per eight-column block (word p = columns 8r + p and 8r + p + 4), with the block's query codes
-// beside them.  G = 4, 8, 16 or 32 by query length (up to 31, 63, 127, 255 bases: the group
-// holds column qlen too), so a warp runs 8 to 1 jobs.  Nothing of a row touches memory.
+// job and a row is one step: lane r of the group holds B eight-column blocks of the row buffer
+// (ksw.cu:310), columns 8 B r on, in registers for the whole job, as the same four int16x2 words of
+// H and four of E per block, with the blocks' query codes beside them.  B G = 4, 8, 16 or 32 by query
+// length (up to 31, 63, 127, 255 bases: the group holds column qlen too), so a warp runs 8 B to B
+// jobs.  Nothing of a row touches memory.
 //
-// One row: every lane runs the block recurrence of g3x_lane16.cuh; the F that enters each block
-// is a max-plus prefix over the group (log2 G shuffles of the blocks' outgoing F, decaying by
-// 8 e_ins per lane); H of the column left of a block comes from the lane before it by one
-// shuffle; the row maximum with its last column is one max over (H << 16 | column) keys; and the
-// trim of end (ksw.cu:390-391) takes the last lane of a ballot over the lanes' non-zero column masks.  Band edges follow g3x_lane16.cuh: columns left of beg hold zeros (the words the
-// band clamp cuts off are zeroed), columns right of end keep their words, column end gets
-// {H(i, end-1), 0}, which the shifted H words of its block hold already.
+// One row: every lane runs the block recurrence of g3x_lane16.cuh; the F that enters each lane
+// is a max-plus prefix over the group (g3x_group.cuh); H of the column left of a lane's first block
+// comes from the lane before it by one shuffle; the row maximum with its last column is one max over
+// (H << 16 | column) keys; and the trim of end (ksw.cu:390-391) takes the last lane of a ballot over
+// the lanes' non-zero column masks.  Band edges follow g3x_lane16.cuh: columns left of beg hold
+// zeros (the words the band clamp cuts off are zeroed), columns right of end keep their words, column
+// end gets {H(i, end-1), 0}, which the shifted H words of its block hold already.
 //
-// What bounds it: latency for small batches (a row is one dependent chain of about 300 cycles,
-// half of it the shuffles of the F prefix), issue slots (about 150 instructions a warp row)
-// beyond a few thousand jobs.
+// What bounds it: latency for small batches -- a warp alone takes 600 cycles over a row's 220
+// dependent-heavy instructions --, the ALU pipe beyond a few thousand jobs (84% busy at 20k jobs).
+// 62 jobs 598 us -> 113, 20k 800 -> 323 against the lane classes.
 #include <cuda_runtime.h>
 #include "g3x_core.h"
 #include "g3x_group.cuh"
@@ -35,6 +35,7 @@ namespace {
 using namespace l16;
 
 constexpr int kBlockWarps = 2;
+constexpr int kOneBlockJobs = 32768;
 
 // Masks by h = clamp(end - first column of the block, -1, 8), entry h + 1: the pair words of
 // the columns left of end and right of end, and the bits of the columns up to end.
@@ -77,7 +78,7 @@ struct GroupJob {
 // next band) overlap the next row's blocks, whose inputs they are not: an iteration starts with
 // row i's blocks and F prefix, then finishes row i - 1's bookkeeping from the reductions issued at
 // its end, and then completes row i within the band that this gives.
-template <int G, bool kSym>
+template <int G, int B, bool kSym>
 __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParams& sp, const PairConst& pc,
                                            const EdgeTable& tab, const uint2* pools, const int32_t* order, int n,
                                            int32_t* queue, int32_t* misfit, int32_t* misfits, int lane,
@@ -89,13 +90,19 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
     unsigned leaders = 0;
 #pragma unroll
     for (int k = 0; k < kGroups; ++k) leaders |= 1u << (k * G);
-    const int col0 = 8 * r;
+    const int col0 = 8 * B * r;
     const int32_t zdrop = sp.zdrop > 0 ? sp.zdrop : 0x7FFFFFFF;
 
     GroupJob J = {};
     J.job = -1;
-    uint32_t H[4] = {0u, 0u, 0u, 0u}, E[4] = {0u, 0u, 0u, 0u};
-    uint32_t qw = 0, tw = 0;      // query codes of the block; target codes of rows 8 (r + G c) ..
+    uint32_t H[B][4], E[B][4];
+    uint32_t qw[B], tw = 0;       // query codes of the blocks; target codes of rows 8 (r + G c) ..
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        qw[b] = 0u;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) H[b][p] = E[b][p] = 0u;
+    }
     uint2 pl = pools[0];          // score pools of row i
     // row i - 1: (maximum << 16 | its last column), its to-end score, and its last lane with
     // non-zero columns with their mask
@@ -110,21 +117,22 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
         // ---- row i: the blocks with F from zero, and the F entering each ----
         RowState rs;
         rs.plo = pl.x; rs.phi = pl.y;
-        BlockA a;
-        uint32_t ne[4], nh[4], h2[4];
-        phase_a<kSym>(H, E, qw, rs, pc, a, ne);
-        rs.fr = (uint32_t)f_entering<G>((int32_t)__viaddmax_s16x2(a.L2[3] << 16, pc.n4, a.L2[3]), r, sp.e_ins);
+        BlockA a[B];
+        uint32_t ne[B][4];
+        int32_t x = 0;                                   // F leaving the lane's blocks
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            phase_a<kSym>(H[b], E[b], qw[b], rs, pc, a[b], ne[b]);
+            const int32_t xb = (int32_t)__viaddmax_s16x2(a[b].L2[3] << 16, pc.n4, a[b].L2[3]);
+            x = b ? __viaddmax_s32(x, decay_hi(sp.e_ins, 1), xb) : xb;
+        }
+        rs.fr = (uint32_t)f_entering<G>(x, r, B * sp.e_ins);
         rs.hlast = 0u;
         // score pools of row i + 1: lane r holds the target codes of rows i0 + 8r .. + 7, i0 the
         // last multiple of 8 G rows
         const int32_t i1 = J.i + 1;
         if ((i1 & (8 * G - 1)) == 0) {
-            const int ch = (i1 >> 4) + (r >> 1);
-            if (ch << 4 < J.tlen) {
-                uint32_t x, nb;
-                load16(d.codes, d.nmask, J.t_off, J.tlen, ch, J.trev, x, nb);
-                tw = (uint32_t)(nibbles16(x, nb) >> ((r & 1) << 5));
-            }
+            if (J.job >= 0) tw = codes8(d.codes, d.nmask, J.t_off, J.tlen, J.trev, i1 + 8 * r);
         }
         // (the funnel shift takes its amount modulo 32)
         const uint32_t t8 = __shfl_sync(kAll, tw, gb | ((i1 >> 3) & (G - 1)));
@@ -145,7 +153,7 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
         // no positive cell, z-drop or the last row; or no job in any group
         const bool stop = J.job >= 0 ? (uint32_t)key < (uint32_t)kNoRow || zstop || J.i >= J.tlen : all_idle;
         if (__any_sync(kAll, stop)) {
-            const int owner = gb + (J.qlen >> 3);             // holds column qlen
+            const int owner = gb + J.qlen / (8 * B);          // holds column qlen
             const int32_t gs = __shfl_sync(kAll, J.gscore, owner & 31), gi = __shfl_sync(kAll, J.max_ie, owner & 31);
             if (stop && J.job >= 0) {
                 if (r == 0) {
@@ -156,7 +164,6 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                     rows += J.i;
                 }
                 J.job = -1;
-                J.tlen = 0;                                    // no more target codes to load
             }
             // refill together once half of the groups are idle: a refill waits for two dependent
             // global loads, and jobs of a class and length come one after another
@@ -179,7 +186,7 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                     c.o_del = sp.o_del; c.e_del = sp.e_del; c.o_ins = sp.o_ins; c.e_ins = sp.e_ins;
                     c.oe_del = sp.oe_del; c.oe_ins = sp.oe_ins; c.zdrop = sp.zdrop;
                     c.w = clamp_w(jb.w, c.qlen, sp.max_sc, sp.end_bonus, sp.o_del, sp.e_del, sp.o_ins, sp.e_ins);
-                    const bool fits = c.qlen < 8 * G && job_fits_int16(c, sp.max_sc);
+                    const bool fits = c.qlen < 8 * B * G && job_fits_int16(c, sp.max_sc);
                     const bool too_long = c.qlen > d.qmax || c.tlen > d.tmax || !fits;
                     const bool outside = !job_in_planes(jb, d.n_bases);
                     if (!fits && misfit) {
@@ -206,27 +213,20 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                         // column t of a block: half t >> 2 of word t & 3
                         const uint32_t b2 = ((c.qlen & 1) ? 0x54u : 0x10u) + ((c.qlen & 4) ? 0x22u : 0u);
                         J.qsel = b2 | (8u | b2 >> 4) * 0x1100u;      // zero-extended by H's sign
-                        // the block's query codes and the first rows' target codes: halves of
-                        // 16-base chunks
-                        const int c0 = (r >> 1) << 4, half = (r & 1) << 5;
-                        uint32_t x, nb;
-                        qw = tw = 0;
-                        if (c0 < c.qlen) {
-                            load16(d.codes, d.nmask, jb.q_off, c.qlen, r >> 1, (jb.flags & G3X_JOB_QREV) != 0, x, nb);
-                            qw = (uint32_t)(nibbles16(x, nb) >> half);
-                        }
-                        if (c0 < c.tlen) {
-                            load16(d.codes, d.nmask, J.t_off, c.tlen, r >> 1, J.trev, x, nb);
-                            tw = (uint32_t)(nibbles16(x, nb) >> half);
-                        }
-                        // row -1 (ksw.cu:317-319)
+                        // the blocks' query codes, the first rows' target codes and row -1
+                        // (ksw.cu:317-319)
+                        tw = codes8(d.codes, d.nmask, J.t_off, c.tlen, J.trev, 8 * r);
 #pragma unroll
-                        for (int p = 0; p < 4; ++p) {
-                            const int j = col0 + p;
-                            const uint32_t lo = j <= c.qlen + 1 ? (uint32_t)init_h(j, c) : 0u;
-                            const uint32_t hi = j + 4 <= c.qlen + 1 ? (uint32_t)init_h(j + 4, c) : 0u;
-                            H[p] = (lo & 0xFFFFu) | (hi << 16);
-                            E[p] = 0u;
+                        for (int b = 0; b < B; ++b) {
+                            qw[b] = codes8(d.codes, d.nmask, jb.q_off, c.qlen, (jb.flags & G3X_JOB_QREV) != 0, col0 + 8 * b);
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) {
+                                const int j = col0 + 8 * b + p;
+                                const uint32_t lo = j <= c.qlen + 1 ? (uint32_t)init_h(j, c) : 0u;
+                                const uint32_t hi = j + 4 <= c.qlen + 1 ? (uint32_t)init_h(j + 4, c) : 0u;
+                                H[b][p] = (lo & 0xFFFFu) | (hi << 16);
+                                E[b][p] = 0u;
+                            }
                         }
                         // the band of row 0: all of [0, qlen)
                         ll = gb + 64; nzl = 1u;
@@ -247,57 +247,71 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
 
         // ---- the band of row i (ksw.cu:388-391, then 335-345) ----
         const int32_t cut = J.i - J.w;
-        const int32_t end = min(min(8 * (ll - gb) + msb32(nzl) + 2, J.i + J.w + 1), J.qlen);
+        const int32_t end = min(min(8 * B * (ll - gb) + msb32(nzl) + 2, J.i + J.w + 1), J.qlen);
         const int32_t h1 = cut <= 0 ? max(J.hv, 0) : 0;
         J.hv -= sp.e_del;
-        const int h = max(min(end - col0, 8), -1) + 1;
-        const uint4 lv = tab.left[h], rv = tab.right[h];
-        const uint32_t left[4] = {lv.x, lv.y, lv.z, lv.w}, right[4] = {rv.x, rv.y, rv.z, rv.w};
-        const uint32_t upto = tab.upto[h];
-
         // ---- the rest of the row: F and H, the row maximum, the new words ----
-        phase_b(a, rs, pc, nh, h2);
-        const uint32_t hl = __shfl_up_sync(kAll, h2[3], 1, G);
-        int32_t kk[8];
+        uint32_t nh[B][4], h2[B][4];
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const uint32_t v = h2[p] & left[p];
-            kk[p] = (int32_t)(v * sp.k16 + (uint32_t)p);
-            kk[p + 4] = (int32_t)prmt((uint32_t)(p + 4), v, 0x7610u);
-        }
-        key = max3_i32(max3_i32(kk[0], kk[1], kk[2]), max3_i32(kk[3], kk[4], kk[5]), max(kk[6], kk[7])) + col0;
-        key = max_of_group<G>(key);
-        nh[0] = prmt(r ? hl : (uint32_t)h1 << 16, h2[3], 0x5432u);
-        // columns beyond end keep their words, column end has E = 0 (ksw.cu:371)
+        for (int b = 0; b < B; ++b) phase_b(a[b], rs, pc, nh[b], h2[b]);
+        const uint32_t hl = __shfl_up_sync(kAll, rs.hlast, 1, G);
+        key = 0;
+        uint32_t nz = 0u;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            H[p] = (nh[p] & ~right[p]) | (H[p] & right[p]);
-            E[p] = (ne[p] & left[p]) | (E[p] & right[p]);
+        for (int b = 0; b < B; ++b) {
+            const int h = max(min(end - col0 - 8 * b, 8), -1) + 1;
+            const uint4 lv = tab.left[h], rv = tab.right[h];
+            const uint32_t left[4] = {lv.x, lv.y, lv.z, lv.w}, right[4] = {rv.x, rv.y, rv.z, rv.w};
+            int32_t kk[8];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint32_t v = h2[b][p] & left[p];
+                kk[p] = (int32_t)(v * sp.k16 + (uint32_t)(8 * b + p));
+                kk[p + 4] = (int32_t)prmt((uint32_t)(8 * b + p + 4), v, 0x7610u);
+            }
+            key = max3_i32(max3_i32(key, kk[0], kk[1]), max3_i32(kk[2], kk[3], kk[4]), max3_i32(kk[5], kk[6], kk[7]));
+            if (b == 0) nh[0][0] = prmt(r ? hl : (uint32_t)h1 << 16, h2[0][3], 0x5432u);
+            // columns beyond end keep their words, column end has E = 0 (ksw.cu:371)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                H[b][p] = (nh[b][p] & ~right[p]) | (H[b][p] & right[p]);
+                E[b][p] = (ne[b][p] & left[p]) | (E[b][p] & right[p]);
+            }
+            nz |= nonzero_mask(H[b], E[b], tab.upto[h]) << (8 * b);
         }
-        const uint32_t nz = nonzero_mask(H, E, upto);
+        key = max_of_group<G>(key + col0);
         const unsigned bal = __ballot_sync(kAll, nz != 0u) & gmask;
         ll = msb32(bal);
         nzl = __shfl_sync(kAll, nz, ll & 31);
         if (d.cells) {
             J.cells += max(end - max(beg, cut), 0);
             const int fl = ffs32(bal) - 1;
-            beg = 8 * (fl - gb) + ffs32(__shfl_sync(kAll, nz, fl & 31)) - 1;
+            beg = 8 * B * (fl - gb) + ffs32(__shfl_sync(kAll, nz, fl & 31)) - 1;
         }
         // to-end score: H(i, qlen - 1) is the H word of column qlen (used in its lane only)
         {
             const bool w2 = (J.qlen & 2) != 0;
-            const int32_t v = (int32_t)prmt(w2 ? H[2] : H[0], w2 ? H[3] : H[1], J.qsel);
+            uint32_t lo = w2 ? H[0][2] : H[0][0], hi = w2 ? H[0][3] : H[0][1];
+#pragma unroll
+            for (int b = 1; b < B; ++b) {
+                const bool mine = ((J.qlen >> 3) & (B - 1)) == b;
+                lo = mine ? (w2 ? H[b][2] : H[b][0]) : lo;
+                hi = mine ? (w2 ? H[b][3] : H[b][1]) : hi;
+            }
+            const int32_t v = (int32_t)prmt(lo, hi, J.qsel);
             gval = end == J.qlen ? v : kNoGscore;
         }
         // the column that the band clamp cuts off in row i + 1 (ksw.cu:338) becomes zero
         const int cc = cut - col0;
         if (__any_sync(kAll, shr_clamp(nz, (uint32_t)cc) & 1u)) {
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const uint32_t keep = cc == p ? 0xFFFF0000u : cc == p + 4 ? 0x0000FFFFu : 0xFFFFFFFFu;
-                H[p] &= keep;
-                E[p] &= keep;
-            }
+            for (int b = 0; b < B; ++b)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    const uint32_t keep = cc == 8 * b + p ? 0xFFFF0000u : cc == 8 * b + p + 4 ? 0x0000FFFFu : 0xFFFFFFFFu;
+                    H[b][p] &= keep;
+                    E[b][p] &= keep;
+                }
         }
         ++J.i;
     }
@@ -305,11 +319,11 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
     idle += (lane == 0 ? (unsigned long long)iters * kGroups : 0ull) - rows;
 }
 
-// d.order null and d.order_off null: jobs 0 .. n in the given order (or d.order's), one warp each;
-// misfit non-null (see run_groups).  Else classes 0-3 of a sorted batch (order_off: [offset,
-// count] pairs), widest first.
-template <bool kSym>
-__global__ void __launch_bounds__(32 * kBlockWarps) group16_kernel(LaunchDesc d, ScoreParams sp, int32_t* misfit,
+// B = 0: jobs 0 .. n in the given order (or d.order's), one warp each; misfit non-null (see
+// run_groups).  Else classes 0-3 of a sorted batch (order_off: [offset, count] pairs), widest first,
+// B blocks a lane.
+template <int B, bool kSym>
+__global__ void __launch_bounds__(32 * kBlockWarps, B == 2 ? 8 : 1) group16_kernel(LaunchDesc d, ScoreParams sp, int32_t* misfit,
                                                                   int32_t* misfits) {
     pdl_trigger();
     __shared__ EdgeTable tab;
@@ -337,15 +351,15 @@ __global__ void __launch_bounds__(32 * kBlockWarps) group16_kernel(LaunchDesc d,
     const int lane = threadIdx.x & 31;
     const PairConst pc = pair_const(sp);
     unsigned long long busy = 0, idle = 0, waves = 0;
-    if (!d.order_off) {
+    if constexpr (B == 0) {
         const int n = d.count ? *d.count : d.n;
-        run_groups<32, kSym>(d, sp, pc, tab, pools, d.order, n, d.queue, misfit, misfits, lane, busy, idle, waves);
+        run_groups<32, 1, kSym>(d, sp, pc, tab, pools, d.order, n, d.queue, misfit, misfits, lane, busy, idle, waves);
     } else {
         const int32_t* oc = d.order_off;
-        run_groups<32, kSym>(d, sp, pc, tab, pools, d.order + oc[6], oc[7], d.queue + 3, nullptr, nullptr, lane, busy, idle, waves);
-        run_groups<16, kSym>(d, sp, pc, tab, pools, d.order + oc[4], oc[5], d.queue + 2, nullptr, nullptr, lane, busy, idle, waves);
-        run_groups<8, kSym>(d, sp, pc, tab, pools, d.order + oc[2], oc[3], d.queue + 1, nullptr, nullptr, lane, busy, idle, waves);
-        run_groups<4, kSym>(d, sp, pc, tab, pools, d.order + oc[0], oc[1], d.queue, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<32 / B, B, kSym>(d, sp, pc, tab, pools, d.order + oc[6], oc[7], d.queue + 3, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<16 / B, B, kSym>(d, sp, pc, tab, pools, d.order + oc[4], oc[5], d.queue + 2, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<8 / B, B, kSym>(d, sp, pc, tab, pools, d.order + oc[2], oc[3], d.queue + 1, nullptr, nullptr, lane, busy, idle, waves);
+        run_groups<4 / B, B, kSym>(d, sp, pc, tab, pools, d.order + oc[0], oc[1], d.queue, nullptr, nullptr, lane, busy, idle, waves);
     }
     if (d.stats) add_warp_stats(d.stats, busy, idle, waves, lane);
     pdl_chain_end();
@@ -367,7 +381,14 @@ void group16_tiles(TileTable& t) {
 
 int launch_group16(const LaunchDesc& d, const ScoreParams& sp, int32_t* misfit, int32_t* misfits,
                    cudaStream_t stream) {
-    auto kern = sp.oe_del == sp.oe_ins ? group16_kernel<true> : group16_kernel<false>;
+    const bool sym = sp.oe_del == sp.oe_ins;
+    // Blocks per lane in a sorted batch: two halve what a row costs beyond its blocks (half the lanes a
+    // job) and take longer over a row.  One against two: 19.8k jobs 376 and 411 us, 39.6k 690 and 634;
+    // right extensions 20k 479 and 449, 40k 897 and 809; seed calls of 40k 1473 and 1360, 60k 2118 and
+    // 1884, chains of 39k seeds 1324 and 1375.
+    auto kern = !d.order_off ? (sym ? group16_kernel<0, true> : group16_kernel<0, false>)
+                : d.n <= kOneBlockJobs ? (sym ? group16_kernel<1, true> : group16_kernel<1, false>)
+                                       : (sym ? group16_kernel<2, true> : group16_kernel<2, false>);
     const int per_sm = resident_blocks(kern, 32 * kBlockWarps, 0);
     const int need = (d.n + kBlockWarps - 1) / kBlockWarps;
     const int full = sm_count() * (per_sm > 0 ? per_sm : 1);

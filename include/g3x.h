@@ -100,7 +100,7 @@ const char *g3x_strerror(int code);
 #define G3X_KERNEL_LANE16  4  /* one job per lane, two cells per int16x2 instruction (jobs whose
                                  scores fit 16 bits) */
 #define G3X_KERNEL_LANE2   5  /* one job per lane, rows i and i+1 in flight together */
-#define G3X_KERNEL_BAND    6  /* one job per warp, the band's row buffer in registers over a window
+#define G3X_KERNEL_BAND    6  /* 8-32 lanes per job, the band's row buffer in registers over a window
                                  of `tile` columns (256, 512 or 1024, 0 = 1024) that slides with
                                  the band; jobs whose band 2w' + 2 exceeds it get TOO_LONG */
 
@@ -184,7 +184,11 @@ typedef struct {
 /* A new context's classes: the int16x2 lane kernel (lanes 1, tile 2, refill 8) for queries up to
    32, 56, 88, 128, 168, 200 and 256 bases, then 32-lane row-parallel groups (tile 9) for longer
    queries and jobs outside the int16 fit.  g3x_autotune replaces them with classes fitted to a
-   batch. */
+   batch.  Until g3x_set_tiles gives classes, the library also chooses beside them: batches up to
+   36,864 jobs (seed-level waves up to 73,728 seeds, and their retry waves) run in an int16x2
+   kernel of 4-32 lanes per job where the scores fit (and with g3x_set_int16 at 1), and the jobs of
+   the last class whose band fits a window of the band kernel run there when max_qlen exceeds
+   256.  Outputs are the same every way. */
 int g3x_get_tiles(g3x_ctx *ctx, g3x_tile_t *h_tiles, int32_t *n);
 int g3x_set_tiles(g3x_ctx *ctx, const g3x_tile_t *h_tiles, int32_t n);
 /* Whether the context's width classes may use the int16x2 lane kernel (1, a new context's
@@ -211,8 +215,8 @@ int g3x_autotune_schedule(g3x_ctx *ctx, int32_t schedule, const g3x_score_t *sco
                           const uint32_t *d_nmask, int64_t n_bases, int32_t max_qlen,
                           int32_t max_tlen, g3x_tile_t *h_tiles, int32_t *n_tiles);
 /* Occupancy counters of the last persistent batch on this context: h_stats[0] = group-rows
-   computed, [1] = group-rows a group waited for the other groups of its warp (warp_batch),
-   [2] = warp batches.  Synchronises the context's device. */
+   computed (lane kernels: row blocks), [1] = group-rows a group waited for the other groups of its
+   warp (warp_batch), [2] = warp batches.  Synchronises the context's device. */
 int g3x_last_stats(g3x_ctx *ctx, uint64_t *h_stats);
 
 /* Per-class kernel timing of the scheduled batches (no counterpart in the reference): with
@@ -433,9 +437,9 @@ int g3x_traceback_pairs(const g3x_opt_t *opt, const g3x_refinfo_t *ref, const g3
    string follow as the traceback stage computes them after ksw_global2 (bwa/src/aux.cu:2831-2860;
    bases as "ACGTN", or "TGCAN" for jobs with G3X_JOB_MDRC): d_nm[k], and the NUL-terminated MD
    at d_md[k * md_stride] (G3X_ERR_TOO_LONG and an empty string when it does not fit;
-   4 (qlen + tlen) + 16 bytes always do).  Scratch: max_tlen x min(max_qlen, 2 max_w + 1) bytes
-   per resident warp (at most 8 GiB, fewer warps beyond), allocated in the context for larger
-   calls; the jobs are ordered by size with the context's scheduling scratch, so calls on one
+   4 (qlen + tlen) + 16 bytes always do).  Scratch per resident warp: 128 bytes x max_tlen, or, when
+   some band or score may not fit the group kernel, max_tlen x min(max_qlen, 2 max_w + 1) x 32 bytes
+   (at most 8 GiB, fewer warps beyond), allocated in the context for larger calls; the jobs are ordered by size with the context's scheduling scratch, so calls on one
    context belong on one stream.  Asynchronous on `stream`. */
 #define G3X_JOB_MDRC 4u   /* MD prints the reverse-strand alphabet "TGCAN" */
 int g3x_ksw_global2_batch(g3x_ctx *ctx, const g3x_score_t *score, const g3x_job_t *d_jobs, int32_t n,

@@ -29,7 +29,7 @@ def band_jobs(n, seed, ws, h0s, qmin=257):
 
 @pytest.mark.parametrize("score", [{}, dict(o_del=5, e_del=2, o_ins=7, e_ins=1), dict(a=3, b=2, o_del=1, e_del=9, o_ins=2, e_ins=5),
                                    dict(zdrop=0)])
-@pytest.mark.parametrize("n", [60, 3500])
+@pytest.mark.parametrize("n", [60, 6000])
 def test_default_context_long_queries(score, n):
     sc = g.default_score(**score)
     for h0s in ((1, 19, 150), (120, 400, 900)):

@@ -1,8 +1,9 @@
 """GPU parity of the int16x2 group-per-job kernel (g3x_group16.cu), which small scheduled batches
 take on a context whose width classes were not set: against the oracle, and for every kind of job
 it may not take against the row-parallel kernel (the general path).  Sizes: queries on both sides
-of every group width (31 | 32, 63 | 64, 127 | 128, 255 | 256), batches on both sides of the limit
-up to which jobs run as they are listed (1024), and one- and two-job batches."""
+of every group width (31 | 32, 63 | 64, 127 | 128, 255 | 256), batches on both sides of the limits
+up to which jobs run as they are listed (4096) and with one block a lane (32768), and one- and
+two-job batches."""
 import numpy as np
 import pytest
 
@@ -51,7 +52,7 @@ def edge_jobs(n, seed, w):
 
 
 @pytest.mark.parametrize("score", list(SCORES))
-@pytest.mark.parametrize("n", [1, 2, 63, 1024, 1025, 6000])
+@pytest.mark.parametrize("n", [1, 2, 63, 4096, 4097, 36000])
 def test_edges_match_oracle(score, n):
     sc = g.default_score(**SCORES[score])
     u8, jobs = edge_jobs(n, 17 + n, 40)
@@ -63,7 +64,7 @@ def test_edges_match_oracle(score, n):
     np.testing.assert_array_equal(grows, rows)
 
 
-@pytest.mark.parametrize("kind,w,units", [(1, 100, 900), (1, 5, 20000), (2, 100, 500), (2, 100, 12000), (2, 13, 12000)])
+@pytest.mark.parametrize("kind,w,units", [(1, 100, 900), (1, 5, 20000), (2, 100, 500), (2, 100, 12000), (2, 13, 12000), (2, 100, 18000)])
 @pytest.mark.parametrize("score", ["bwa", "uneven"])
 def test_generated_jobs_match_oracle(kind, w, units, score):
     sc = g.default_score(**SCORES[score])
@@ -78,7 +79,7 @@ def test_generated_jobs_match_oracle(kind, w, units, score):
     np.testing.assert_array_equal(out, ref)
 
 
-@pytest.mark.parametrize("n", [200, 3000])
+@pytest.mark.parametrize("n", [200, 9000, 40000])
 def test_refused_and_misfit_jobs_as_on_the_general_path(n):
     sc = g.default_score()
     u8, jobs = edge_jobs(n, 5, 40)
