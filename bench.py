@@ -608,9 +608,9 @@ def run_cfg5_workload(args, ws, rank):
 
 
 # DRAM bytes (read + write) per launch of the dominant kernel of each workload below, from ncu
-# captures of these workloads (global_kernel: 0.427 GB read + 1.010 GB written; sw_kernel<16>:
-# 18.9 MB read, nothing written back but the outputs)
-GLOBAL_DRAM_BYTES = 1_436_724_000
+# captures of these workloads (global16_kernel: 19.3 MB read + 109.7 MB written for 60k of the pairs,
+# scaled to 200k; sw_kernel<16>: 18.9 MB read, nothing written back but the outputs)
+GLOBAL_DRAM_BYTES = 430_220_000
 SW_DRAM_BYTES = 18_913_024
 GLOBAL_JOBS = 200000
 GLOBAL_DESC = ("ksw_global2 with backtrack over 200k synthetic region pairs as the traceback stage issues "
@@ -747,8 +747,8 @@ def run_global_workload(args, ws, rank):
                      "unit": "GCUPS", "frac": round(gcups / max(ws, 1) / peak_gcups, 4),
                      "traffic": GLOBAL_DRAM_BYTES,
                      "note": "cells per second of the global kernel against the int-ALU cells/s peak (8 ops per cell); "
-                             "traffic: DRAM bytes read + written by one global_kernel launch of this workload "
-                             "(an ncu capture of it): the direction bytes"},
+                             "traffic: DRAM bytes read + written by one global16_kernel launch of this workload "
+                             "(an ncu capture of 60k of its pairs, scaled): the direction bits"},
         "cpu_baseline": None if cpu_t is None else {
             "value": round(cells / cpu_t / 1e9, 4), "unit": "GCUPS", "cores": threads, "kind": "reference",
             "sample": "whole rank-0 workload, one pass, the reference's own ksw_global2"},
