@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128) lane16_kernel(LaunchDesc d, ScoreParams s
         busy32 += nblk;
         kmax32 += kmax;
 
-        // ---- the row's blocks: masked first block, middle blocks two at a time, masked last block ----
+        // ---- the row's blocks: masked first block, middle blocks three at a time, masked last block ----
         uint32_t mF, mL;
         row_blocks<kSym, kCells>(P, lane, r, pc, ge, nblk, kmax, any_single, mF, mL);
 

@@ -267,37 +267,42 @@ G3X_HD void block_mid(const Planes& P, int at, int32_t kb, RowState& r, const Pa
     block_max(h2, kb, r);
 }
 
-// Two consecutive blocks strictly inside the row, the second only when `second` (else nothing of
-// it is stored and the row state stays as the first block leaves it).  The F-independent
-// phases of both blocks come first, so the two blocks' instructions interleave.
-template <bool kSym>
-G3X_HD void block_mid2(const Planes& P, int at, int32_t kb, bool second, RowState& r, const PairConst& pc) {
-    const uint4 hq0 = P.H[at], eq0 = P.E[at], hq1 = P.H[at + 32], eq1 = P.E[at + 32];
-    const uint32_t qw0 = P.qn[at], qw1 = P.qn[at + 32];
-    BlockA a0, a1;
-    uint32_t ne0[4], ne1[4];
-    {
-        const uint32_t H2[4] = {hq0.x, hq0.y, hq0.z, hq0.w}, E2[4] = {eq0.x, eq0.y, eq0.z, eq0.w};
-        phase_a<kSym>(H2, E2, qw0, r, pc, a0, ne0);
+// N consecutive blocks strictly inside the row, the first `have` (>= 1) of them this lane's (nothing of
+// the others is stored and the row state stays as the last of its blocks leaves it).  The
+// F-independent phases of all blocks come first, so the blocks' instructions interleave: a warp waits
+// for its dependent DPX steps (1.1-1.3 cycles per issued instruction), and shared memory holds too few
+// warps to cover them, while registers are left over.  N = 3 against 2: 990k jobs in learned order 5.24
+// and 5.00 ms, 198k 1.26 and 1.10.  Four at a time measured 5.20, five 4.98, three without tails of two
+// and one 5.26.
+template <int N, bool kSym>
+G3X_HD void block_mids(const Planes& P, int at, int32_t kb, int have, RowState& r, const PairConst& pc) {
+    BlockA a[N];
+    uint32_t ne[N][4];
+#pragma unroll
+    for (int b = 0; b < N; ++b) {
+        // (no read beyond the row's last block, which follows the lane's `have`)
+        const int ab = at + 32 * (b < 2 || b <= have ? b : 1);
+        const uint4 hq = P.H[ab], eq = P.E[ab];
+        const uint32_t H2[4] = {hq.x, hq.y, hq.z, hq.w}, E2[4] = {eq.x, eq.y, eq.z, eq.w};
+        phase_a<kSym>(H2, E2, P.qn[ab], r, pc, a[b], ne[b]);
     }
-    {
-        const uint32_t H2[4] = {hq1.x, hq1.y, hq1.z, hq1.w}, E2[4] = {eq1.x, eq1.y, eq1.z, eq1.w};
-        phase_a<kSym>(H2, E2, qw1, r, pc, a1, ne1);
+    uint32_t nh[N][4], h2[N][4], fr[N], hl[N];
+    RowState rb = r;
+#pragma unroll
+    for (int b = 0; b < N; ++b) {
+        phase_b(a[b], rb, pc, nh[b], h2[b]);
+        fr[b] = rb.fr;
+        hl[b] = rb.hlast;
     }
-    uint32_t nh0[4], h20[4], nh1[4], h21[4];
-    phase_b(a0, r, pc, nh0, h20);
-    RowState r1 = r;
-    phase_b(a1, r1, pc, nh1, h21);
-    P.E[at] = make_uint4(ne0[0], ne0[1], ne0[2], ne0[3]);
-    P.H[at] = make_uint4(nh0[0], nh0[1], nh0[2], nh0[3]);
-    block_max(h20, kb, r);
-    if (second) {
-        P.E[at + 32] = make_uint4(ne1[0], ne1[1], ne1[2], ne1[3]);
-        P.H[at + 32] = make_uint4(nh1[0], nh1[1], nh1[2], nh1[3]);
-        r.fr = r1.fr;
-        r.hlast = r1.hlast;
-        block_max(h21, kb + 1, r);
-    }
+#pragma unroll
+    for (int b = 0; b < N; ++b)
+        if (b == 0 || b < have) {
+            P.E[at + 32 * b] = make_uint4(ne[b][0], ne[b][1], ne[b][2], ne[b][3]);
+            P.H[at + 32 * b] = make_uint4(nh[b][0], nh[b][1], nh[b][2], nh[b][3]);
+            r.fr = fr[b];
+            r.hlast = hl[b];
+            block_max(h2[b], kb + b, r);
+        }
 }
 
 // The first block of a row with two or more blocks: the words left of beg are zeroed on load.
@@ -551,8 +556,8 @@ G3X_HD void row_end(LaneJob& J, const Planes& P, int lane, const RowState& r, co
 // All blocks of one row of one lane, in the order the kernel runs them.
 // The blocks of one row of one lane as the kernel's warp runs them: kmax (>= nblk) is the most
 // blocks any lane of the warp has in this row, and every lane walks the same iterations, doing
-// only its own blocks: the first (masked), the middle ones two at a time (one alone when an odd
-// number of them is left for the warp), the last (masked).  Returns the first block's and the
+// only its own blocks: the first (masked), the middle ones three at a time (then two or one when the
+// warp has that many left), the last (masked).  Returns the first block's and the
 // last block's non-zero column masks for row_end in mF, mL.  any_single: some lane of the warp
 // has a one-block row (nblk == 1).
 template <bool kSym, bool kCells>
@@ -563,8 +568,12 @@ G3X_HD void row_blocks(const Planes& P, int lane, RowState& r, const PairConst& 
     const int at0 = (kb0 << 5) + lane;              // its uint4 index in the lane-interleaved planes
     if (nblk > 1) mF = block_first<kSym, kCells>(P, at0, kb0, r, pc, ge);
     int k = 1, at = at0 + 32;
-    for (; k + 1 < kmax - 1; k += 2, at += 64)
-        if (k < nblk - 1) block_mid2<kSym>(P, at, kb0 + k, k + 1 < nblk - 1, r, pc);
+    for (; k + 2 < kmax - 1; k += 3, at += 96)
+        if (k < nblk - 1) block_mids<3, kSym>(P, at, kb0 + k, nblk - 1 - k, r, pc);
+    if (k + 1 < kmax - 1) {
+        if (k < nblk - 1) block_mids<2, kSym>(P, at, kb0 + k, nblk - 1 - k, r, pc);
+        k += 2; at += 64;
+    }
     if (k < kmax - 1 && k < nblk - 1) block_mid<kSym>(P, at, kb0 + k, r, pc);
     if (nblk > 0)
         mL = block_last<kSym>(P, at0 + ((nblk - 1) << 5), kb0 + nblk - 1, nblk == 1, any_single, r, pc, ge);

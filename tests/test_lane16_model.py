@@ -49,3 +49,21 @@ def test_lane16_model_asymmetric_gaps():
     ok = status == 0
     assert ok.mean() > 0.9
     assert (out[ok] == ref[ok]).all() and (cells[ok] == rcells[ok]).all()
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+def test_lane16_model_every_block_count(extra):
+    """Rows of 1 to 31 blocks, at a block's edge and one column to either side: every number of middle
+    blocks, and so every remainder of the three that run together."""
+    wl = g.synth(2, 1500, seed=77 + extra, w=300, unrelated=0.1)
+    sc = g.default_score()
+    jobs = wl.jobs.copy()
+    want = 8 * (1 + np.arange(jobs.size) % 31) + extra
+    jobs["qlen"] = np.minimum(jobs["qlen"], want)
+    out, cells, status = nat.emu16_extend(jobs, wl.u8, sc)
+    ref, rcells, _ = nat.oracle_extend(jobs, wl.u8, sc)
+    assert np.unique((jobs["qlen"][status == 0] + 7) // 8).size >= 25
+    assert set(np.unique(status)) <= {0, -3}
+    ok = status == 0
+    assert ok.mean() > 0.9
+    assert (out[ok] == ref[ok]).all() and (cells[ok] == rcells[ok]).all()
