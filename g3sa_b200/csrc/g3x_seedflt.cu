@@ -137,6 +137,7 @@ __global__ void sfl_keep_kernel(int32_t a, const g3x_read_t* __restrict__ reads,
                 s.score = sc < 0 ? s.len * a : sc;
             }
             const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+            __syncwarp();                               // (the ballot alone does not order memory)
             if (keep) seeds[beg + k + __popc(kept & ((1u << lane) - 1u))] = s;
             k += __popc(kept);
             __syncwarp();                               // (a later chain may hold the same slots)

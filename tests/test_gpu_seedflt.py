@@ -56,3 +56,17 @@ def test_gpu_flt_seeds_rejects_bad_reads():
     keep = np.ones(len(wl.chains), bool)
     keep[mine] = False
     assert np.array_equal(c1["n"][keep], c2["n"][keep])
+
+
+def test_gpu_flt_seeds_compacts_long_chains_in_place():
+    """Chains of more than a warp's 32 seeds with dropped seeds among them: a step's seeds are all read
+    before its kept ones move down over them, whose slots other lanes of the step read."""
+    wl = synth_chains(60, seed=12, read_lens=(3000, 4500), div=0.05, spurious=0.2)
+    c1, s1, sw1, _ = nat.oracle_flt_seeds(wl, nat.opt_from_score(g.default_score(), w=100), 60)
+    n0 = wl.chains["n"]
+    assert (n0 > 32).sum() >= 20 and ((c1["n"] > 32) & (c1["n"] < n0)).sum() >= 10
+    for _ in range(3):
+        c2, s2, sw2, st = run_flt(wl, g.default_opt(w=100), 60)
+        assert (st == 0).all()
+        assert np.array_equal(sw1, sw2) and np.array_equal(c1["n"], c2["n"])
+        assert kept(c1, s1) == kept(c2, s2)
