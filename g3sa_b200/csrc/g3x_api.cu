@@ -38,10 +38,10 @@ GlobalScratch& ctx_global(g3x_ctx* ctx) { return ctx->global; }
 SwScratch& ctx_sw(g3x_ctx* ctx) { return ctx->sw; }
 
 
-int pair_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, int classes, cudaStream_t st, const int32_t** order,
+int pair_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, int classes, bool rest, cudaStream_t st, const int32_t** order,
                const int32_t** range) {
     int rc = alloc_sched(ctx->sched, n);
-    if (rc || (rc = sort_pairs(ctx->sched, jobs, n, classes, st))) return rc;
+    if (rc || (rc = sort_pairs(ctx->sched, jobs, n, classes, rest, st))) return rc;
     *order = ctx->sched.order;
     *range = ctx->sched.bucket_oc;
     return G3X_OK;

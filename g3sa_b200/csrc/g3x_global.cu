@@ -304,7 +304,8 @@ extern "C" int g3x_ksw_global2_batch(g3x_ctx* ctx, const g3x_score_t* score, con
     const cudaStream_t st = (cudaStream_t)stream;
     d.range = nullptr;
     d.order = nullptr;
-    if (!direct && (rc = pair_order(ctx, d_jobs, n, groups ? kGlobalGroupClasses : 0, st, &d.order, &d.range))) return rc;
+    if (!direct && (rc = pair_order(ctx, d_jobs, n, groups ? kGlobalGroupClasses : 0, lanes, st, &d.order, &d.range)))
+        return rc;
     if (cudaMemsetAsync(gs.queue, 0, (kGlobalGroupClasses + 1) * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
     if (groups) {
         GlobalDesc g = d;

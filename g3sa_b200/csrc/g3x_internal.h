@@ -392,11 +392,12 @@ struct SwScratch {
 };
 SwScratch& ctx_sw(g3x_ctx* ctx);
 // The context's order of global-alignment jobs (its scheduling scratch): by band class, class k of
-// `classes` for up to 16 << k columns 2w + 1, the rest last; in a class by decreasing row count and
-// row width.  range: [offset, count] of each class and of the rest, in device memory.
-int pair_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, int classes, cudaStream_t st, const int32_t** order,
+// `classes` for up to 16 << k columns 2w + 1, the rest last (rest false: in the widest class); in a
+// class by decreasing row count and row width.  range: [offset, count] of each class and of the rest, in
+// device memory.
+int pair_order(g3x_ctx* ctx, const g3x_job_t* jobs, int n, int classes, bool rest, cudaStream_t st, const int32_t** order,
                const int32_t** range);
-int sort_pairs(SchedScratch& s, const g3x_job_t* jobs, int n, int classes, cudaStream_t st);
+int sort_pairs(SchedScratch& s, const g3x_job_t* jobs, int n, int classes, bool rest, cudaStream_t st);
 void free_chain_scratch(ChainScratch& w);
 
 // Learned cost model state (device buffers; g3x_model.cu).

@@ -111,15 +111,17 @@ __global__ void scatter_kernel(const int32_t* __restrict__ bin, int n, int32_t* 
 }
 
 // Global-alignment jobs: the band class, then rows (the groups' classes), or rows (four bins per
-// doubling) and the widest row (the lane kernel's).
-__global__ void pair_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int classes, int32_t* __restrict__ bin,
-                                int32_t* __restrict__ hist) {
+// doubling) and the widest row (the lane kernel's).  rest 0: the lane kernel is not launched, because
+// every job within the call's bounds fits a group; a wider one is beyond them, and the widest class,
+// whose kernel refuses it, takes it.
+__global__ void pair_bin_kernel(const g3x_job_t* __restrict__ jobs, int n, int classes, int rest,
+                                int32_t* __restrict__ bin, int32_t* __restrict__ hist) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const g3x_job_t jb = jobs[k];
     const int w = min(max(jb.w, 0), (int)max(jb.qlen, jb.tlen));
     int c = 0;
-    while (c < classes && 2 * w + 1 > 16 << c) ++c;
+    while (c < classes - !rest && 2 * w + 1 > 16 << c) ++c;
     const float lr = log2f(1.0f + (float)jb.tlen);
     const int rb = min(max((int)((16.0f - lr) * (kSchedRowBins / 16.0f)), 0), kSchedRowBins - 1);
     const int wb = kSchedWidthBins - 1 - min((min((int)jb.qlen, 2 * w + 1) + 7) >> 3, kSchedWidthBins - 1);
@@ -151,11 +153,11 @@ int batch_max_w(const g3x_job_t* jobs, int n, const ScoreParams& sp, int32_t* d_
     return G3X_OK;
 }
 
-int sort_pairs(SchedScratch& s, const g3x_job_t* jobs, int n, int classes, cudaStream_t st) {
+int sort_pairs(SchedScratch& s, const g3x_job_t* jobs, int n, int classes, bool rest, cudaStream_t st) {
     const int nbins = (classes + 1) * kLevels;
     if (cudaMemsetAsync(s.hist, 0, nbins * sizeof(int32_t), st) != cudaSuccess) return G3X_ERR_CUDA;
     const int tb = 256, nb = (n + tb - 1) / tb;
-    pair_bin_kernel<<<nb, tb, 0, st>>>(jobs, n, classes, s.bin, s.hist);
+    pair_bin_kernel<<<nb, tb, 0, st>>>(jobs, n, classes, rest, s.bin, s.hist);
     scan_kernel<<<1, 1024, 0, st>>>(s.hist, nbins, s.cursor, s.bucket_oc, classes + 1);
     scatter_kernel<<<nb, tb, 0, st>>>(s.bin, n, s.cursor, s.order, nullptr, nullptr);
     return cudaPeekAtLastError() == cudaSuccess ? G3X_OK : G3X_ERR_CUDA;

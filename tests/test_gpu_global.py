@@ -190,3 +190,41 @@ def test_gpu_global_group_widths(n, score):
         np.testing.assert_array_equal(nm2, nm1)
         md = d_md.cpu().numpy().reshape(n, md_stride)
         assert [bytes(md[k]).split(b"\0")[0].decode() for k in range(n)] == md1
+
+
+@pytest.mark.parametrize("n", [1000, 1025, 5000])
+@pytest.mark.parametrize("mq,mt,mw", [(250, 260, 100), (120, 120, 300), (250, 260, 400)])
+def test_gpu_global_writes_every_refused_pair(n, mq, mt, mw):
+    """Jobs beyond the call's bounds or past the planes, their bands on both sides of the widest group's
+    (127), with the lane kernel launched (bounds that allow wider bands) and without, unsorted and
+    sorted: every output of each is written, whatever the caller's buffers held."""
+    import torch
+    cj, u8 = nat.global_jobs(n, 41 + n, max_len=250, ws=(5, 20, 100))
+    jobs = gpu_jobs(cj)
+    k = np.random.default_rng(n).permutation(n)[:200]
+    jobs["w"][k[:60]] = np.resize([127, 128, 200, 60000, 0x7FFFFFFF, -1], 60)
+    jobs["q_off"][k[60:90]] = len(u8) + 7
+    jobs["t_off"][k[90:120]] = 0xFFFFFFF0
+    jobs["w"][k[75:105]] = 60000
+    q_end, t_end = jobs["q_off"].astype(np.int64) + jobs["qlen"], jobs["t_off"].astype(np.int64) + jobs["tlen"]
+    outside = (q_end > len(u8)) | (t_end > len(u8))
+    bad = outside | (jobs["qlen"] > mq) | (jobs["tlen"] > mt) | (jobs["w"] > mw) | (jobs["w"] < 0)
+    stride, md_stride = 520, 64
+    codes, nmask = g.pack_planes(u8)
+    out = [torch.full((n * w,), 77, dtype=torch.int32, device="cuda") for w in (1, stride, 1, 1, 1)]
+    d_md = torch.full((n * md_stride,), 77, dtype=torch.uint8, device="cuda")
+    c = g.Context(0)
+    c.global_batch(g.default_score(), to_dev(jobs), n, to_dev(codes), to_dev(nmask), mq, mt, mw, out[0], out[1], stride,
+                   out[2], out[3], d_nm=out[4], d_md=d_md, md_stride=md_stride, n_bases=len(u8))
+    torch.cuda.synchronize()
+    score, _, n_cigar, status, nm = [t.cpu().numpy() for t in out]
+    c.close()
+    np.testing.assert_array_equal(status[bad], np.where(outside, g.G3X_ERR_INVALID, g.G3X_ERR_TOO_LONG)[bad])
+    assert (score[bad] == 0).all() and (n_cigar[bad] == 0).all() and (nm[bad] == 0).all()
+    assert (d_md.cpu().numpy().reshape(n, md_stride)[bad, 0] == 0).all()
+    taken = cj.copy()
+    taken["w"] = jobs["w"]
+    s1, _, n1, _ = nat.oracle_global(taken[~bad], u8, g.default_score(), stride)
+    assert np.isin(status[~bad], (g.G3X_OK, g.G3X_ERR_TOO_LONG)).all()      # (an MD beyond its stride)
+    np.testing.assert_array_equal(score[~bad], s1)
+    np.testing.assert_array_equal(n_cigar[~bad], n1)
