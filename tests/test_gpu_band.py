@@ -8,6 +8,7 @@ import pytest
 
 import g3sa_b200 as g
 from tests import native as nat
+from tests.gpu_util import to_dev
 from tests.test_gpu_group16 import run
 
 pytestmark = pytest.mark.gpu
@@ -72,7 +73,6 @@ def test_band_kernel_small_queries_and_tails(kernel_tile):
     jobs["tlen"] = np.minimum(jobs["tlen"], rng.choice([0, 1, 16, 17, 200, 700], len(jobs)))
     ref, cells, rows = nat.oracle_extend(jobs, u8, sc)
     import torch
-    from tests.gpu_util import to_dev
     c = g.Context(0)
     n = len(jobs)
     codes, nmask = g.pack_planes(u8)
@@ -87,3 +87,32 @@ def test_band_kernel_small_queries_and_tails(kernel_tile):
     np.testing.assert_array_equal(gcells.cpu().numpy(), cells)
     np.testing.assert_array_equal(grows.cpu().numpy(), rows)
     c.close()
+
+
+@pytest.mark.parametrize("n", [9000, 17000])
+@pytest.mark.parametrize("kernel,tile", [(g.KERNEL_AUTO, 0), (g.KERNEL_BAND, 512), (g.KERNEL_BAND, 256)])
+def test_negative_bands_beside_wide_ones(n, kernel, tile):
+    """A warp's jobs share the registers that the widest of its bands needs (two and four jobs a warp from
+    8,000 and 16,000 jobs on); a band below 0, which has no cells, changes nothing for the others."""
+    import torch
+    sc = g.default_score()
+    u8, base = band_jobs(340, 5, (100, 120) if tile == 256 else (100, 240), (19, 150))
+    base["tlen"] = np.minimum(base["tlen"], np.random.default_rng(1).choice([300, 420, 600], len(base)))
+    ref, cells, rows = nat.oracle_extend(base, u8, sc)
+    jobs = np.resize(base, n)
+    at, neg = np.arange(n) % len(base), np.arange(n) % 7 == 3
+    jobs["w"][neg] = np.where(np.arange(n)[neg] % 2, -1, -5)
+    codes, nmask = g.pack_planes(u8)
+    out = torch.full((n, 6), -777, dtype=torch.int32, device="cuda")
+    status, gcells, grows = (torch.full((n,), 99, dtype=torch.int32, device="cuda") for _ in range(3))
+    c = g.Context(0)
+    c.extend_batch(sc, to_dev(jobs), n, to_dev(codes), to_dev(nmask), out, status, int(jobs["qlen"].max()),
+                   int(jobs["tlen"].max()), schedule=g.SCHED_SORTED, kernel=kernel, tile=tile, d_cells=gcells,
+                   d_rows=grows)
+    torch.cuda.synchronize()
+    c.close()
+    assert (status.cpu().numpy() == 0).all()
+    ok = ~neg
+    np.testing.assert_array_equal(out.cpu().numpy()[ok], ref[at[ok]])
+    np.testing.assert_array_equal(gcells.cpu().numpy()[ok], cells[at[ok]])
+    np.testing.assert_array_equal(grows.cpu().numpy()[ok], rows[at[ok]])
