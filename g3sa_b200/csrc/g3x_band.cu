@@ -362,6 +362,8 @@ __global__ void __launch_bounds__(64) band_kernel(LaunchDesc d, ScoreParams sp) 
                         refuse(d, job, G3X_OK);
                         d.out[job] = g3x_ext_t{c.h0, 0, 0, 0, -1, 0};
                     }
+                } else if (c.w < 0) {
+                    if (r == 0) finish_empty_band(d, job, c);
                 } else {
                     J.job = job;
                     J.c = c;
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(64) band_kernel(LaunchDesc d, ScoreParams sp) 
         if (!have) continue;
         jobs_run += __popc(have);
         // the narrowest registers that hold the warp's bands: a row costs about 11 instructions a column
-        const int cols = 2 * (int)__reduce_max_sync(kAll, (unsigned)max(J.c.w, 0)) + 1;   // (a band below 0: no cells)
+        const int cols = 2 * __reduce_max_sync(kAll, J.c.w) + 1;
 #define G3X_BAND(R) run_band<G, (R), kSym>(d, sp, J, pools, lane, rows_run)
         if constexpr (W == 256) {
             if (cols <= 64) G3X_BAND(64 / G);

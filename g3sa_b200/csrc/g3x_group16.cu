@@ -200,6 +200,8 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                             if (d.cells) d.cells[job] = 0;
                             if (d.rows) d.rows[job] = 0;
                         }
+                    } else if (c.w < 0) {
+                        if (r == 0) finish_empty_band(d, job, c);
                     } else {
                         fresh = true;
                         J.job = job;

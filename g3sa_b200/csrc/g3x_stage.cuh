@@ -249,6 +249,17 @@ __device__ bool stage_job(int job, const LaunchDesc& d, const ScoreParams& sp,
     return true;
 }
 
+// A band below 0, which the clamp of ksw.cu:321-329 keeps, has no cell: row 0 begins at column -w, is
+// empty and ends the job, with a to-end score of 0 if that column is the query's end (ksw.cu:338-345,
+// 372-376).  For kernels whose rows take the band's first column from the row itself.
+__device__ __forceinline__ void finish_empty_band(const LaunchDesc& d, int job, const JobConst& c) {
+    const bool ends = c.qlen == -(int64_t)c.w;
+    d.out[job] = g3x_ext_t{c.h0, 0, 0, ends ? 1 : 0, ends ? 0 : -1, 0};
+    d.status[job] = G3X_OK;
+    if (d.cells) d.cells[job] = 0;
+    if (d.rows) d.rows[job] = 1;
+}
+
 // Programmatic dependent launch in the width-class kernels.  pdl_trigger, first thing in the
 // kernel, lets the class kernel queued after this one on the stream start at once (its blocks
 // take the SMs this kernel's blocks leave as they run out of jobs).  pdl_chain_end, last thing:

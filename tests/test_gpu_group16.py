@@ -99,3 +99,49 @@ def test_refused_and_misfit_jobs_as_on_the_general_path(n):
     assert ((got[1] != 0) == (want[1] != 0)).all()
     for a, b in zip(got[:1] + got[2:4], want[:1] + want[2:4]):
         np.testing.assert_array_equal(a, b)
+
+
+def negative_band_results(jobs):
+    """What the row loop gives a band below 0: an empty row 0 from column -w on, which ends the job; a
+    to-end score of 0 when that column is the query's end.  Returns (ext[n, 6], rows[n])."""
+    ran = jobs["tlen"] > 0
+    ends = ran & (jobs["qlen"] == -jobs["w"].astype(np.int64))
+    out = np.zeros((len(jobs), 6), np.int32)
+    out[:, 0], out[:, 3], out[:, 4] = jobs["h0"], ends, np.where(ends, 0, -1)
+    return out, ran.astype(np.int32)
+
+
+def test_negative_band_rule_matches_oracle():
+    """(the oracle, like the reference, writes before its row for bands below -1)"""
+    u8, jobs = edge_jobs(2000, 3, 40)
+    jobs["w"] = -1
+    ref, cells, rows = nat.oracle_extend(jobs, u8, g.default_score())
+    want, want_rows = negative_band_results(jobs)
+    np.testing.assert_array_equal(want, ref)
+    np.testing.assert_array_equal(want_rows, rows)
+    assert (cells == 0).all() and (want[:, 4] == 0).any()
+
+
+@pytest.mark.parametrize("kernel", [g.KERNEL_AUTO, g.KERNEL_ROWPAR, g.KERNEL_BAND])
+@pytest.mark.parametrize("n", [63, 4096, 9000])
+def test_negative_bands(n, kernel):
+    """Negative bands among others, queries that end where such a band's row 0 begins and empty queries
+    among them: in the group kernel as they are listed and sorted, the row-parallel and the band
+    kernel."""
+    u8, jobs = edge_jobs(n, 23 + n, 40)
+    rng = np.random.default_rng(n)
+    neg = rng.random(n) < 0.3
+    to_end = -np.maximum(jobs["qlen"].astype(np.int32), 1)
+    jobs["w"][neg] = np.where(rng.random(n) < 0.5, to_end, rng.choice([-1, -2, -30, -60000], n))[neg]
+    want, want_rows = negative_band_results(jobs)
+    assert (want[neg, 4] == 0).any()
+    sc = g.default_score()
+    out, status, cells, rows, _ = run(u8, jobs, sc, kernel=kernel)
+    assert (status == 0).all()
+    np.testing.assert_array_equal(out[neg], want[neg])
+    np.testing.assert_array_equal(rows[neg], want_rows[neg])
+    assert (cells[neg] == 0).all()
+    ref, ref_cells, ref_rows = nat.oracle_extend(jobs[~neg], u8, sc)
+    np.testing.assert_array_equal(out[~neg], ref)
+    np.testing.assert_array_equal(rows[~neg], ref_rows)
+    np.testing.assert_array_equal(cells[~neg], ref_cells)
