@@ -38,7 +38,8 @@ __device__ __forceinline__ int row_level(float log2_rows) {
 __device__ __forceinline__ int sched_key(const g3x_job_t& jb, const ScoreParams& sp, const TileTable& tt,
                                          bool has_pred, float pred) {
     const int w = clamp_w(jb.w, jb.qlen, sp.max_sc, sp.end_bonus, sp.o_del, sp.e_del, sp.o_ins, sp.e_ins);
-    const int wide = jb.qlen < 2 * w + 1 ? jb.qlen : 2 * w + 1;
+    const int cols = w < 0 ? 0 : 2 * w + 1;            // (a negative band has no cells)
+    const int wide = jb.qlen < cols ? jb.qlen : cols;
     int b = tt.n - 1;
     for (int t = 0; t < tt.n; ++t)
         if (tt.width[t] >= jb.qlen) { b = t; break; }

@@ -122,12 +122,12 @@ def test_negative_band_rule_matches_oracle():
     assert (cells == 0).all() and (want[:, 4] == 0).any()
 
 
-@pytest.mark.parametrize("kernel", [g.KERNEL_AUTO, g.KERNEL_ROWPAR, g.KERNEL_BAND])
-@pytest.mark.parametrize("n", [63, 4096, 9000])
+@pytest.mark.parametrize("kernel,n", [(k, n) for k in (g.KERNEL_AUTO, g.KERNEL_ROWPAR, g.KERNEL_BAND) for n in (63, 4096, 9000)]
+                         + [(g.KERNEL_AUTO, 40000)])
 def test_negative_bands(n, kernel):
     """Negative bands among others, queries that end where such a band's row 0 begins and empty queries
     among them: in the group kernel as they are listed and sorted, the row-parallel and the band
-    kernel."""
+    kernel, and the lane classes (40,000), whose sort keys hold the width of the widest row."""
     u8, jobs = edge_jobs(n, 23 + n, 40)
     rng = np.random.default_rng(n)
     neg = rng.random(n) < 0.3
