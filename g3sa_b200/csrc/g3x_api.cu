@@ -199,6 +199,7 @@ static int launch_last(const LaunchDesc& d, const ScoreParams& sp, int32_t* queu
     LaunchDesc r = d;
     r.queue = queue;
     r.split = d.qmax > 256;
+    if (r.split) r.warp_batch = 0;    // the row-parallel kernel passes the band kernel's jobs by in its per-group refill
     int rc = launch_rowpar(r, sp, st);
     if (!r.split) return rc;
     r.kernel = kKernelBand;

@@ -49,7 +49,7 @@ struct LaunchDesc {
     int32_t pdl;           // class kernels: 1 = launched as a programmatic dependent of the
                            // class kernel before it on the stream (launch_class_kernel)
     int32_t split;         // 1: the band kernel and the row-parallel kernel share the jobs by their
-                           // bands (band_window): each skips what is not its own
+                           // bands (band_window): each skips what is not its own (needs warp_batch 0)
     int32_t retry;         // a seed-level retry wave: few of its n jobs, a device-side count
     int64_t n_bases;       // bases the planes hold: jobs reaching past them are refused
     int64_t step_limit;    // plain (rolling) kernel: per-job step bound, 0 = the default bound

@@ -116,3 +116,29 @@ def test_negative_bands_beside_wide_ones(n, kernel, tile):
     np.testing.assert_array_equal(out.cpu().numpy()[ok], ref[at[ok]])
     np.testing.assert_array_equal(gcells.cpu().numpy()[ok], cells[at[ok]])
     np.testing.assert_array_equal(grows.cpu().numpy()[ok], rows[at[ok]])
+
+
+def test_tuned_last_class_runs_each_job_once():
+    """The last class of a tuned table may refill a warp's groups together (warp_batch), a path that takes
+    every job; it is tuned when the sample holds queries beyond the bound given for it.  Longer jobs
+    then: every result, and the row and cell counts, as from one run of each job."""
+    import torch
+    sc = g.default_score()
+    u8, jobs = band_jobs(600, 11, (40, 100), (19, 150))
+    jobs["qlen"][::4] = 180
+    ref, cells, rows = nat.oracle_extend(jobs, u8, sc)
+    codes, nmask = g.pack_planes(u8)
+    d = to_dev(jobs), len(jobs), to_dev(codes), to_dev(nmask)
+    mq, mt = int(jobs["qlen"].max()), int(jobs["tlen"].max())
+    c = g.Context(0)
+    for _ in range(4):
+        c.autotune(sc, *d, 200, mt)
+        out = torch.full((len(jobs), 6), -777, dtype=torch.int32, device="cuda")
+        status, gcells, grows = (torch.full((len(jobs),), 99, dtype=torch.int32, device="cuda") for _ in range(3))
+        c.extend_batch(sc, *d, out, status, mq, mt, schedule=g.SCHED_SORTED, d_cells=gcells, d_rows=grows)
+        torch.cuda.synchronize()
+        assert (status.cpu().numpy() == 0).all()
+        np.testing.assert_array_equal(out.cpu().numpy(), ref)
+        np.testing.assert_array_equal(grows.cpu().numpy(), rows)
+        np.testing.assert_array_equal(gcells.cpu().numpy(), cells)
+    c.close()
