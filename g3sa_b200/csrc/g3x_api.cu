@@ -27,7 +27,7 @@ struct g3x_ctx {
     int cls_timed[g3x::kMaxBuckets];        // 1 when the last batch recorded class k
     int64_t step_limit;                     // g3x_set_step_limit (0: the kernels' own bound)
     int no_int16;                           // g3x_set_int16(ctx, 0): width classes in int32 only
-    int tiles_set;                          // width classes given by g3x_set_tiles
+    int tiles_set;                          // width classes given by g3x_set_tiles or fitted by g3x_autotune
 };
 
 namespace g3x {
@@ -300,8 +300,8 @@ constexpr int64_t kGroupJobs = 36864, kGroupSeeds = 73728;
 // 3k 449 against 566, 5k 543 against 577, 10k 813 against 601.
 constexpr int64_t kDirectJobs = 4096, kDirectSeeds = 5120;
 
-// Contexts with width classes of their own (g3x_set_tiles), in int32 or with class timing keep to
-// them.
+// Contexts with width classes of their own (g3x_set_tiles, g3x_autotune), in int32 or with class timing
+// keep to them.
 static bool groups_allowed(const g3x_ctx* ctx) { return !ctx->tiles_set && !ctx->no_int16 && !ctx->timing; }
 
 // Runs a batch (or with base.order a wave of at most base.n jobs) through the group-per-job
@@ -692,6 +692,7 @@ int g3x_autotune_schedule(g3x_ctx* ctx, int32_t schedule, const g3x_score_t* sco
         t.width[t.n] = 0x7FFFFFFF; t.lanes[t.n] = 32; t.tile[t.n] = 9; t.warp_batch[t.n] = 0; t.refill[t.n] = 1;
         ++t.n;
         ctx->tiles = t;
+        ctx->tiles_set = 1;
     }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);

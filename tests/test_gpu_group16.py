@@ -145,3 +145,32 @@ def test_negative_bands(n, kernel):
     np.testing.assert_array_equal(out[~neg], ref)
     np.testing.assert_array_equal(rows[~neg], ref_rows)
     np.testing.assert_array_equal(cells[~neg], ref_cells)
+
+
+@pytest.mark.parametrize("kind,units", [(2, 3000), (4, 400)])
+def test_autotuned_classes_run_as_the_same_classes_set(kind, units):
+    """g3x_autotune's table in its context and handed to another through g3x_set_tiles: the same jobs per
+    class, the same results; and a context without either sorts the batch into the groups' classes."""
+    import torch
+    wl = g.synth(kind, units, seed=9, w=60, unrelated=0.2 if kind == 2 else 0.0)
+    codes, nmask = wl.planes()
+    d = to_dev(wl.jobs), wl.n, to_dev(codes), to_dev(nmask)
+    mq, mt = int(wl.jobs["qlen"].max()), int(wl.jobs["tlen"].max())
+    sc = g.default_score()
+    ref, _, _ = nat.oracle_extend(wl.jobs, wl.u8, sc)
+    tuned, same, plain = g.Context(0), g.Context(0), g.Context(0)
+    same.set_tiles(tuned.autotune(sc, *d, mq, mt))
+    jobs = []
+    for c in (tuned, same, plain):
+        out = torch.zeros((wl.n, 6), dtype=torch.int32, device="cuda")
+        status = torch.full((wl.n,), 9, dtype=torch.int32, device="cuda")
+        c.extend_batch(sc, *d, out, status, mq, mt, schedule=g.SCHED_SORTED)
+        torch.cuda.synchronize()
+        assert (status.cpu().numpy() == 0).all()
+        np.testing.assert_array_equal(out.cpu().numpy(), ref)
+        jobs.append([k for _, k in c.class_times()])
+    for c in (tuned, same, plain):
+        c.close()
+    assert jobs[0] == jobs[1] and sum(jobs[0]) == wl.n
+    if kind == 2:
+        assert jobs[2] != jobs[0]
