@@ -368,8 +368,11 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     SchedScratch& sched = *res.sched;
     // A retry wave holds the few jobs whose band was too narrow (their count stays on the device):
     // in groups it lasts 0.1 ms where a lane class of a handful of jobs lasts 0.5.
-    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= kGroupSeeds))
-        return run_grouped(d, sp, sched, res.queue, d.n <= kDirectSeeds, st);
+    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= kGroupSeeds)) {
+        LaunchDesc g = d;
+        g.stats = res.stats;
+        return run_grouped(g, sp, sched, res.queue, d.n <= kDirectSeeds, st);
+    }
     int rc = w->learned && ctx->model.active
                  ? schedule_jobs_learned(sched, d.jobs, d.n, d.codes, d.nmask, d.n_bases, ctx->model.params, sp,
                                          ctx->tiles, st, d.order, d.count)
