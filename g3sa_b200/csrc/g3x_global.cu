@@ -285,9 +285,12 @@ extern "C" int g3x_ksw_global2_batch(g3x_ctx* ctx, const g3x_score_t* score, con
     }
     const bool direct = groups && !lanes && n <= kDirectPairs;
     if (groups) {
-        gblocks = std::min(global16_blocks(), (n + kGlobal16Warps - 1) / kGlobal16Warps);
+        // (for the whole device whatever n is: a call captured after a smaller one within the same bounds
+        // must find its scratch)
+        gblocks = global16_blocks();
         while (gblocks > 1 && (int64_t)gblocks * kGlobal16Warps * zgroup > cap) gblocks = gblocks / 2;
         need = std::max(need, (int64_t)gblocks * kGlobal16Warps * zgroup);
+        gblocks = std::min(gblocks, (n + kGlobal16Warps - 1) / kGlobal16Warps);
     }
     GlobalScratch& gs = ctx_global(ctx);
     if (gs.bytes < need || !gs.queue) {

@@ -228,3 +228,45 @@ def test_gpu_global_writes_every_refused_pair(n, mq, mt, mw):
     assert np.isin(status[~bad], (g.G3X_OK, g.G3X_ERR_TOO_LONG)).all()      # (an MD beyond its stride)
     np.testing.assert_array_equal(score[~bad], s1)
     np.testing.assert_array_equal(n_cigar[~bad], n1)
+
+
+def test_gpu_global_captured_after_a_smaller_call():
+    """Scratch depends on the call's bounds, not on its pairs (up to the 1,024 that a context's order
+    scratch always holds): a call of the same bounds is captured into a graph after a smaller one, and
+    the smaller one's graph still runs after it."""
+    import torch
+    n, small = 1000, 40
+    cj, u8 = nat.global_jobs(n, 77, max_len=200, ws=(5, 20))
+    codes, nmask = g.pack_planes(u8)
+    d_jobs, d_codes, d_nmask = to_dev(gpu_jobs(cj)), to_dev(codes), to_dev(nmask)
+    mq, mt = int(cj["qlen"].max()), int(cj["tlen"].max())
+    stride = mq + mt + 2
+    s1, c1, n1, _ = nat.oracle_global(cj, u8, g.default_score(), stride)
+    c = g.Context(0)
+    out = [torch.zeros(n * k, dtype=torch.int32, device="cuda") for k in (1, stride, 1, 1)]
+
+    def call(k):
+        c.global_batch(g.default_score(), d_jobs, k, d_codes, d_nmask, mq, mt, 20, out[0], out[1], stride, out[2], out[3],
+                       stream=st)
+
+    st = torch.cuda.Stream()
+    call(small)
+    st.synchronize()
+    graphs = []
+    for k in (small, n):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=st):
+            call(k)
+    for gr, k in zip(reversed(graphs), (n, small)):
+        for t in out:
+            t.fill_(77)
+        gr.replay()
+        torch.cuda.synchronize()
+        score, cig, nc, status = [t.cpu().numpy() for t in out]
+        assert (status[:k] == 0).all()
+        np.testing.assert_array_equal(score[:k], s1[:k])
+        np.testing.assert_array_equal(nc[:k], n1[:k])
+        cig = cig.view(np.uint32).reshape(n, stride)
+        assert all(np.array_equal(cig[j, :n1[j]], c1[j, :n1[j]]) for j in range(k))
+    del graphs
+    c.close()
