@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(64) band_kernel(LaunchDesc d, ScoreParams sp) 
 #undef G3X_BAND
     }
     if (d.stats) {
-        if (r == 0) atomicAdd(d.stats + 0, rows_run);
-        if (lane == 0) atomicAdd(d.stats + 2, jobs_run);
+        if (r == 0 && rows_run) atomicAdd(d.stats + 0, rows_run);
+        if (lane == 0 && jobs_run) atomicAdd(d.stats + 2, jobs_run);
     }
     pdl_chain_end();
 }

@@ -175,7 +175,7 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                 if (lane == 0) first = atomicAdd(queue, __popc(want));
                 first = __shfl_sync(kAll, first, 0);
                 exhausted = first + __popc(want) >= n;
-                ++waves;
+                waves += first < n;
                 const int slot = first + __popc(want & ((1u << gb) - 1u));
                 bool fresh = false;
                 if (J.job < 0 && slot < n) {

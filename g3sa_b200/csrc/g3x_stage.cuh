@@ -281,11 +281,10 @@ __device__ __forceinline__ void add_warp_stats(unsigned long long* stats, unsign
         busy += __shfl_xor_sync(0xFFFFFFFFu, busy, o);
         idle += __shfl_xor_sync(0xFFFFFFFFu, idle, o);
     }
-    if (lane == 0) {
-        atomicAdd(stats + 0, busy);
-        atomicAdd(stats + 1, idle);
-        atomicAdd(stats + 2, waves);
-    }
+    // (a warp that ran no job adds nothing: a class without jobs has thousands of those, and their adds to
+    // one address take 5 us)
+    const unsigned long long v = lane == 0 ? busy : lane == 1 ? idle : waves;
+    if (lane < 3 && v) atomicAdd(stats + lane, v);
 }
 
 }  // namespace g3x
