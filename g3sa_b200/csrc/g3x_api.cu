@@ -284,17 +284,35 @@ static int launch_classes(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParam
 }
 
 // The group-per-job kernel or the width classes.  A lane class lasts as long as its longest job
-// (0.5-1.1 ms at 250 bases, whatever its job count) and then costs 5.2-8 ns a job; a group costs
-// 14-22 ns a job and 0.1 ms at least.  Measured on batches of uneven left and right extensions, group
-// against lanes: 62 jobs 113 and 606 us, 9.9k jobs 259 and 1063, 19.8k 376 and 1065, 39.6k 634 and
-// 1079, 79k 1155 and 1115; right extensions of 1-150 bases: 20k 449 and 892, 40k 809 and 926, 60k 1177
-// and 946; w = 30: 39.6k 537 and 554, 59k 745 and 558.  So batches up to 36k jobs take the groups; from
-// there on narrow bands gain nothing, and the order a caller chose (by length or learned), which the
-// groups ignore, keeps deciding.  A seed call (left wave, right wave and their retry waves) pays the
-// lanes' latency more often: 20k seeds 846 and 2171 us, 40k 1360 and 2310, 60k 1884 and 2356, so its
-// waves take them up to 72k.  Waves that run side by side (the seed stream's) fill the lanes together
-// and count together.
+// (0.5-1.1 ms at 250 bases and wide bands, whatever its job count) and then costs 5.2-8 ns a job; a group
+// costs 14-22 ns a job and 0.1 ms at least.  Measured on batches of uneven left and right extensions at
+// w = 100, group against lanes: 62 jobs 113 and 606 us, 9.9k jobs 259 and 1063, 19.8k 376 and 1065, 39.6k
+// 634 and 1079, 79k 1155 and 1115.  So batches up to 36k jobs take the groups at most; from there on they
+// gain little, and the order a caller chose (by length or learned), which the groups ignore, keeps
+// deciding.  A seed call (left wave, right wave and their retry waves) pays the lanes' latency more
+// often: 20k seeds 846 and 2171 us, 40k 1360 and 2310, 60k 1884 and 2356, so its waves take them up to
+// 72k at most.  Waves that run side by side (the seed stream's) fill the lanes together and count
+// together.
+//
+// A lane's time falls with its row, the narrower of band and query, a group's (sized by the query)
+// does not, so the line falls with the band w and the longest query q of the batch.  Where group and
+// lanes cross, in thousands: queries of 1-150 bases w = 5 13.5, 10 15.7, 20 19.7, 30 24, 50 29, 75 39,
+// 100 44 (36k at w = 10 495 and 306 us); the same cut to 100 bases w = 5 22, 20 32, to 60 w = 5 33; left
+// and right flanks of 100-250-base reads (most far shorter than the longest) w = 5 19.5, 10 23, 20
+// 28.5, 30 39, 50 over 50; seeds of 250-base reads w = 5 20, 10 24, 20 28.5, 40 47, 60 57, 100 70 (72k at
+// w = 10 2059 and 1446 us), of 150-base reads w = 5 37, 10 43, 30 58, of 100-base reads w = 5 57, 10 66.
 constexpr int64_t kGroupJobs = 36864, kGroupSeeds = 73728;
+static int64_t group_jobs(int64_t w, int32_t qmax) {
+    const int64_t q = std::min(std::max(qmax, 1), 256), b = std::max<int64_t>(w, 0);
+    return std::min(kGroupJobs, q < 192 ? (1600 + 55 * b) * 1000 / q : 16000 + 480 * b);
+}
+static int64_t group_seeds(int64_t w, int32_t qmax) {
+    const int64_t q = std::min(std::max(qmax, 1), 256), b = std::max<int64_t>(w, 0);
+    return std::min(kGroupSeeds, (4200 + 135 * b) * 1000 / q);
+}
+// A batch's bands are known to the device alone; but targets cut as the reference cuts them (the query
+// and a gap of at most 2 w more, aux.cu:168-205) show the band in the call's bounds.
+static int64_t bounds_band(const LaunchDesc& d) { return std::max((d.tmax - d.qmax) / 2, 0); }
 // Up to here a job takes a warp in the order given: 62 jobs 113 us against 126 sorted into classes
 // (three launches less), 2k 186 against 205, 4k 227 against 240, 6k 273 against 252; seed calls of
 // 3k 449 against 566, 5k 543 against 577, 10k 813 against 601.
@@ -344,7 +362,7 @@ static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams
     int rc = alloc_sched(ctx->sched, base.n);
     if (rc) return rc;
     if (learned && (!ctx->model.params || !ctx->model.trained)) return G3X_ERR_NOT_TRAINED;
-    if (groups_allowed(ctx) && base.n <= kGroupJobs) {
+    if (groups_allowed(ctx) && base.n <= group_jobs(bounds_band(base), base.qmax)) {
         LaunchDesc d = base;
         d.stats = ctx->d_stats;
         if (cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), st) != cudaSuccess) return G3X_ERR_CUDA;
@@ -368,7 +386,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     SchedScratch& sched = *res.sched;
     // A retry wave holds the few jobs whose band was too narrow (their count stays on the device):
     // in groups it lasts 0.1 ms where a lane class of a handful of jobs lasts 0.5.
-    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= kGroupSeeds)) {
+    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= group_seeds(w->band, d.qmax))) {
         LaunchDesc g = d;
         g.stats = res.stats;
         return run_grouped(g, sp, sched, res.queue, d.n <= kDirectSeeds, st);
@@ -385,7 +403,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
 }
 
 // Whether a seed-level call goes through the width classes, and how to run its waves.
-static int seed_waves(g3x_ctx* ctx, const g3x_batch_opts_t* opts, const LaunchDesc& proto, int64_t n,
+static int seed_waves(g3x_ctx* ctx, const g3x_opt_t& opt, const g3x_batch_opts_t* opts, const LaunchDesc& proto, int64_t n,
                       ClassWave* cw, WaveRunner* wr, const WaveRunner** out) {
     *out = nullptr;
     if (!(proto.persistent && proto.kernel == kKernelRowpar && opts->kernel == G3X_KERNEL_AUTO &&
@@ -399,6 +417,7 @@ static int seed_waves(g3x_ctx* ctx, const g3x_batch_opts_t* opts, const LaunchDe
     cw->learned = learned;
     cw->res = nullptr;
     cw->at_once = 1;
+    cw->band = opt.w;
     wr->run = run_class_wave;
     wr->user = cw;
     *out = wr;
@@ -831,7 +850,7 @@ int g3x_extend_seeds(g3x_ctx* ctx, const g3x_opt_t* opt, const g3x_seed_t* d_see
     g3x::ClassWave cw;
     g3x::WaveRunner wr;
     const g3x::WaveRunner* runner = nullptr;
-    if ((rc = g3x::seed_waves(ctx, opts, proto, n, &cw, &wr, &runner))) return rc;
+    if ((rc = g3x::seed_waves(ctx, *opt, opts, proto, n, &cw, &wr, &runner))) return rc;
     return g3x::extend_seeds(ctx->seeds, *opt, sp, d_seeds, n, d_codes, d_nmask, d_regs, d_status,
                              proto, (cudaStream_t)stream, runner);
 }
@@ -856,7 +875,7 @@ int g3x_extend_seeds_stream(g3x_ctx* ctx, const g3x_opt_t* opt, const g3x_seed_t
     g3x::ClassWave cw;
     g3x::WaveRunner wr;
     const g3x::WaveRunner* runner = nullptr;
-    if ((rc = g3x::seed_waves(ctx, opts, proto, chunk > 0 ? chunk : 65536, &cw, &wr, &runner))) return rc;
+    if ((rc = g3x::seed_waves(ctx, *opt, opts, proto, chunk > 0 ? chunk : 65536, &cw, &wr, &runner))) return rc;
     return g3x::extend_seeds_stream(ctx->stream, *opt, sp, h_seeds, n,
                                     h_codes, h_nmask, n_bases, h_regs, h_status, chunk, proto, runner);
 }

@@ -315,6 +315,7 @@ struct ClassWave {
     bool learned;
     const ClassRes* res;
     int32_t at_once;    // waves of this size that run side by side
+    int32_t band;       // the call's band (g3x_opt_t.w)
 };
 int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaStream_t st);
 

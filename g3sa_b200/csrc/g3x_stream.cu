@@ -162,7 +162,8 @@ int extend_seeds_stream(StreamScratch& ss, const g3x_opt_t& opt, const ScorePara
         s.pending = -1;
         if (!runner) continue;
         res[l] = ClassRes{&s.sched, s.queue, nullptr, nullptr, nullptr, nullptr};
-        cw[l] = ClassWave{cw0->ctx, cw0->learned, &res[l], (int32_t)std::min<int64_t>(nchunks, kStreamLanes)};
+        cw[l] = ClassWave{cw0->ctx, cw0->learned, &res[l], (int32_t)std::min<int64_t>(nchunks, kStreamLanes),
+                          cw0->band};
         wr[l] = WaveRunner{runner->run, &cw[l]};
     }
     const int64_t total_code_words = (n_bases + 15) / 16, total_mask_words = (n_bases + 31) / 32;

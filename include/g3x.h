@@ -184,11 +184,12 @@ typedef struct {
 /* A new context's classes: the int16x2 lane kernel (lanes 1, tile 2, refill 8) for queries up to
    32, 56, 88, 128, 168, 200 and 256 bases, then 32-lane row-parallel groups (tile 9) for longer
    queries and jobs outside the int16 fit.  g3x_autotune replaces them with classes fitted to a
-   batch.  Until g3x_set_tiles or g3x_autotune gives classes, the library also chooses beside them: batches up to
-   36,864 jobs (seed-level waves up to 73,728 seeds, and their retry waves) run in an int16x2
-   kernel of 4-32 lanes per job where the scores fit (and with g3x_set_int16 at 1), and the jobs of
-   the last class whose band fits a window of the band kernel run there when max_qlen exceeds
-   256.  Outputs are the same every way. */
+   batch.  Until g3x_set_tiles or g3x_autotune gives classes, the library also chooses beside them:
+   batches up to 36,864 jobs (seed-level waves up to 73,728 seeds, and their retry waves; fewer where
+   bands are narrow and queries long, as the call's bounds and g3x_opt_t.w show them) run in an
+   int16x2 kernel of 4-32 lanes per job where the scores fit (and with g3x_set_int16 at 1), and the
+   jobs of the last class whose band fits a window of the band kernel run there when max_qlen
+   exceeds 256.  Outputs are the same every way. */
 int g3x_get_tiles(g3x_ctx *ctx, g3x_tile_t *h_tiles, int32_t *n);
 int g3x_set_tiles(g3x_ctx *ctx, const g3x_tile_t *h_tiles, int32_t n);
 /* Whether the context's width classes may use the int16x2 lane kernel (1, a new context's

@@ -1,5 +1,5 @@
 """GPU parity of the int16x2 group-per-job kernel (g3x_group16.cu), which small scheduled batches
-take on a context whose width classes were not set: against the oracle, and for every kind of job
+take on a context whose width classes were not given: against the oracle, and for every kind of job
 it may not take against the row-parallel kernel (the general path).  Sizes: queries on both sides
 of every group width (31 | 32, 63 | 64, 127 | 128, 255 | 256), batches on both sides of the limits
 up to which jobs run as they are listed (4096) and with one block a lane (32768), and one- and
@@ -64,15 +64,18 @@ def test_edges_match_oracle(score, n):
     np.testing.assert_array_equal(grows, rows)
 
 
-@pytest.mark.parametrize("kind,w,units", [(1, 100, 900), (1, 5, 20000), (2, 100, 500), (2, 100, 12000), (2, 13, 12000), (2, 100, 18000)])
+@pytest.mark.parametrize("kind,w,units", [(1, 100, 900), (1, 5, 11000), (1, 5, 20000), (2, 100, 500), (2, 100, 12000), (2, 13, 9000),
+                                          (2, 13, 12000), (2, 100, 18000)])
 @pytest.mark.parametrize("score", ["bwa", "uneven"])
 def test_generated_jobs_match_oracle(kind, w, units, score):
+    """Batches on both sides of the line that falls with the band: beyond it the lane classes run them."""
     sc = g.default_score(**SCORES[score])
     wl = g.synth(kind, units, seed=units + w, w=w, unrelated=0.3)
     ref, cells, rows = nat.oracle_extend(wl.jobs, wl.u8, sc)
     out, status, gcells, grows, stats = run(wl.u8, wl.jobs, sc)
     assert (status == 0).all()
-    assert stats[0] == rows.sum()                      # the group kernel counts rows, the lane kernels row blocks
+    # the group kernel counts rows, the lane kernels row blocks
+    assert (stats[0] == rows.sum()) == ((kind, w, units) not in ((1, 5, 20000), (2, 13, 12000)))
     np.testing.assert_array_equal(out, ref)
     np.testing.assert_array_equal(gcells, cells)
     np.testing.assert_array_equal(grows, rows)
@@ -177,22 +180,24 @@ def test_autotuned_classes_run_as_the_same_classes_set(kind, units):
         assert jobs[2] != jobs[0]
 
 
-@pytest.mark.parametrize("units", [700, 9000])
-def test_counters_of_seed_calls(units):
+@pytest.mark.parametrize("units,w", [(700, 100), (9000, 100), (60000, 100), (15000, 10), (60000, 10)])
+def test_counters_of_seed_calls(units, w):
     """A seed-level call's waves add to the context's occupancy counters in groups too (direct and
-    sorted), as in the lane classes."""
+    sorted), as in the lane classes, which take narrow bands from fewer seeds on."""
     import torch
-    wl = g.synth(2, units, seed=3, w=100, unrelated=0.2)
+    wl = g.synth(2, units, seed=3, w=w, unrelated=0.2)
     codes, nmask = wl.planes()
     ds = g.device_seeds(wl.seeds)
     regs = torch.zeros(len(ds) * g.REG_DT.itemsize, dtype=torch.uint8, device="cuda")
     status = torch.zeros(len(ds), dtype=torch.int32, device="cuda")
     _, _, rows = nat.oracle_extend(wl.jobs, wl.u8, g.default_score())
     c = g.Context(0)
-    c.extend_seeds(g.default_opt(w=100), to_dev(ds), len(ds), to_dev(codes), to_dev(nmask), regs, status,
+    c.extend_seeds(g.default_opt(w=w), to_dev(ds), len(ds), to_dev(codes), to_dev(nmask), regs, status,
                    int(wl.seeds["l_query"].max()), int((wl.seeds["rmax1"] - wl.seeds["rmax0"]).max()))
     torch.cuda.synchronize()
     got = c.last_stats()[0]
     c.close()
-    # the left and right extensions are the workload's jobs, but for the right ones' seed scores
-    assert 0.5 * rows.sum() < got < 2 * rows.sum()
+    # the left and right extensions are the workload's jobs, but for the right ones' seed scores; the
+    # lane kernels count a row's blocks (three and more at w = 10)
+    lanes = (units, w) == (60000, 10)
+    assert rows.sum() * (2 if lanes else 0.5) < got < rows.sum() * (8 if lanes else 1.5)
