@@ -310,6 +310,12 @@ static int64_t group_seeds(int64_t w, int32_t qmax) {
     const int64_t q = std::min(std::max(qmax, 1), 256), b = std::max<int64_t>(w, 0);
     return std::min(kGroupSeeds, (4200 + 135 * b) * 1000 / q);
 }
+// A retry wave holds the jobs whose band was too narrow; their count stays on the device.  In groups a
+// few of them last 0.1 ms, in a lane class 0.5, but they are 3% of a call's seeds a side at w = 5, 1.5% at
+// 6 and 7, 0.4% at 8 and less from there on.  Retry waves in groups and in lanes: 400k seeds w = 10 2.49
+// and 2.71 ms, 8 2.37 and 2.51, 6 2.40 and 2.48, 5 2.43 and 2.38; 1M w = 10 5.94 and 6.18, 8 5.57 and
+// 5.70, 5 6.17 and 5.25; 2M w = 10 11.49 and 11.64.
+static int64_t retry_seeds(int64_t w) { return w < 8 ? 1 << 18 : 1 << 22; }
 // A batch's bands are known to the device alone; but targets cut as the reference cuts them (the query
 // and a gap of at most 2 w more, aux.cu:168-205) show the band in the call's bounds.
 static int64_t bounds_band(const LaunchDesc& d) { return std::max((d.tmax - d.qmax) / 2, 0); }
@@ -384,9 +390,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     g3x_ctx* ctx = w->ctx;
     const ClassRes res = w->res ? *w->res : ctx_res(ctx);
     SchedScratch& sched = *res.sched;
-    // A retry wave holds the few jobs whose band was too narrow (their count stays on the device):
-    // in groups it lasts 0.1 ms where a lane class of a handful of jobs lasts 0.5.
-    if (groups_allowed(ctx) && (d.retry || (int64_t)d.n * w->at_once <= group_seeds(w->band, d.qmax))) {
+    if (groups_allowed(ctx) && (d.retry ? d.n <= retry_seeds(w->band) : (int64_t)d.n * w->at_once <= group_seeds(w->band, d.qmax))) {
         LaunchDesc g = d;
         g.stats = res.stats;
         return run_grouped(g, sp, sched, res.queue, d.n <= kDirectSeeds, st);

@@ -41,9 +41,10 @@ def test_seeds_retry_counts_match_oracle():
     assert (regs["tries_left"] == 2).sum() + (regs["tries_right"] == 2).sum() > 10
 
 
-@pytest.mark.parametrize("w", [100, 6])
-def test_seeds_fresh_vs_oracle(w):
-    wl = g.synth(2, 20000, seed=515 + w, w=w, unrelated=0.2)
+@pytest.mark.parametrize("w,units", [(100, 20000), (6, 20000), (5, 270000), (8, 270000)])
+def test_seeds_fresh_vs_oracle(w, units):
+    """(270,000 seeds: the retry waves in lane classes at w = 5, in groups at w = 8)"""
+    wl = g.synth(2, units, seed=515 + w, w=w, unrelated=0.2)
     opt_cpu = nat.opt_from_score(g.default_score(), w=w)
     ref = nat.oracle_seeds(wl.seeds, wl.u8, opt_cpu)
     regs, status = run_seeds(wl.u8, wl.seeds, g.default_opt(w=w))
