@@ -323,6 +323,17 @@ static int64_t bounds_band(const LaunchDesc& d) { return std::max((d.tmax - d.qm
 // (three launches less), 2k 186 against 205, 4k 227 against 240, 6k 273 against 252; seed calls of
 // 3k 449 against 566, 5k 543 against 577, 10k 813 against 601.
 constexpr int64_t kDirectJobs = 4096, kDirectSeeds = 5120;
+// Queries beyond 256 bases only pass the group kernel, and reach the last class's kernels as they come
+// or longest first.  The order costs 10-40 us, pays where jobs wait for a warp, which the registers of
+// the window that their bands need decide, and puts the longest jobs of a batch that starts at once on
+// the same SMs.  As they come and sorted, ms: w = 50 3,000 jobs 3.4 and 4.3; w = 100 1,500 3.8 and 3.5,
+// 3,000 4.1 and 5.2, 4,000 4.4 and 5.3; w = 150 1,500 3.6 and 4.0, 3,000 4.7 and 4.2, 4,000 5.4 and 4.3;
+// w = 254 1,500 4.4 and 5.5, 3,000 5.8 and 5.1; w = 300 300 3.29 and 3.31, 1,500 5.6 and 4.9, 3,000 7.4
+// and 5.3; w = 500 300 3.9 and 3.9, 1,500 7.4 and 6.4, 3,000 10.3 and 7.3, 4,000 12.2 and 9.2.
+// (The windows change at 128 and 256; a target's insertions show as up to an eighth more band.)
+static int64_t direct_jobs(int64_t w, int32_t qmax, int64_t most) {
+    return qmax <= 256 || w < 144 ? most : w < 288 ? 2048 : 512;
+}
 
 // Contexts with width classes of their own (g3x_set_tiles, g3x_autotune), in int32 or with class timing
 // keep to them.
@@ -372,7 +383,8 @@ static int run_scheduled(g3x_ctx* ctx, const LaunchDesc& base, const ScoreParams
         LaunchDesc d = base;
         d.stats = ctx->d_stats;
         if (cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), st) != cudaSuccess) return G3X_ERR_CUDA;
-        return run_grouped(d, sp, ctx->sched, ctx->d_queue, base.n <= kDirectJobs, st);
+        return run_grouped(d, sp, ctx->sched, ctx->d_queue,
+                           base.n <= direct_jobs(bounds_band(base), base.qmax, kDirectJobs), st);
     }
     rc = learned && ctx->model.active
              ? schedule_jobs_learned(ctx->sched, base.jobs, base.n, base.codes, base.nmask, base.n_bases,
@@ -393,7 +405,7 @@ int run_class_wave(void* user, const LaunchDesc& d, const ScoreParams& sp, cudaS
     if (groups_allowed(ctx) && (d.retry ? d.n <= retry_seeds(w->band) : (int64_t)d.n * w->at_once <= group_seeds(w->band, d.qmax))) {
         LaunchDesc g = d;
         g.stats = res.stats;
-        return run_grouped(g, sp, sched, res.queue, d.n <= kDirectSeeds, st);
+        return run_grouped(g, sp, sched, res.queue, d.n <= direct_jobs(w->band, d.qmax, kDirectSeeds), st);
     }
     int rc = w->learned && ctx->model.active
                  ? schedule_jobs_learned(sched, d.jobs, d.n, d.codes, d.nmask, d.n_bases, ctx->model.params, sp,

@@ -142,3 +142,32 @@ def test_tuned_last_class_runs_each_job_once():
         np.testing.assert_array_equal(grows.cpu().numpy(), rows)
         np.testing.assert_array_equal(gcells.cpu().numpy(), cells)
     c.close()
+
+
+@pytest.mark.parametrize("w,n,ordered", [(60, 3000, False), (200, 2000, False), (200, 2100, True), (500, 512, False), (500, 600, True)])
+def test_long_jobs_of_wide_bands_stay_ordered(w, n, ordered):
+    """Long jobs that wait for a warp are sorted (the jobs per class show the sort: all in the rest of the
+    groups' classes), those that start at once are taken as they come; the bounds show the band."""
+    import torch
+    sc = g.default_score()
+    wl = g.synth(4, n, seed=w, w=w, unrelated=0.0)
+    jobs = wl.jobs[wl.jobs["qlen"] > 256]
+    jobs = np.resize(jobs, n)
+    jobs["qlen"] = np.minimum(jobs["qlen"], 700)
+    jobs["tlen"] = np.minimum(jobs["tlen"], jobs["qlen"] + 2 * w)
+    ref, _, _ = nat.oracle_extend(jobs, wl.u8, sc)
+    codes, nmask = wl.planes()
+    d_codes, d_nmask, mq = to_dev(codes), to_dev(nmask), int(jobs["qlen"].max())
+    c = g.Context(0)
+    seen = []
+    for k in (513 if w == 500 else 2049 if w == 200 else 4097, n):        # a sorted batch first
+        more = np.resize(jobs, k)
+        out = torch.zeros((k, 6), dtype=torch.int32, device="cuda")
+        status = torch.full((k,), 9, dtype=torch.int32, device="cuda")
+        c.extend_batch(sc, to_dev(more), k, d_codes, d_nmask, out, status, mq, mq + 2 * w, schedule=g.SCHED_SORTED)
+        torch.cuda.synchronize()
+        assert (status.cpu().numpy() == 0).all()
+        np.testing.assert_array_equal(out.cpu().numpy(), np.resize(ref, (k, 6)))
+        seen.append(c.class_times()[4][1])
+    c.close()
+    assert seen[0] > 0 and (seen[1] == n) == ordered and (ordered or seen[1] == seen[0])
