@@ -67,13 +67,6 @@ __device__ __forceinline__ bool band_fits(const JobConst& c, int32_t max_sc, int
     return 2 * c.w + 2 <= W && (int64_t)c.qlen * max_sc + (c.h0 > 0 ? c.h0 : 0) < (1 << 21);
 }
 
-__device__ __forceinline__ void refuse(const LaunchDesc& d, int job, int32_t status) {
-    d.out[job] = g3x_ext_t{0, 0, 0, 0, 0, 0};
-    d.status[job] = status;
-    if (d.cells) d.cells[job] = 0;
-    if (d.rows) d.rows[job] = 0;
-}
-
 // F entering each lane of a group: exclusive prefix over the lanes of the F leaving each lane's R
 // columns, dec = R e_ins.  A lane that a shuffle leaves alone meets its own value, decayed.
 template <int G>
@@ -350,20 +343,12 @@ __global__ void __launch_bounds__(64) band_kernel(LaunchDesc d, ScoreParams sp) 
                 c.w = clamp_w(jb.w, c.qlen, sp.max_sc, sp.end_bonus, sp.o_del, sp.e_del, sp.o_ins, sp.e_ins);
                 // the checks of stage_job (M = min(H + S, 256 H) needs h0 >= 0 or h0 <= -max_score),
                 // and a band that fits the window
-                const bool bad_h0 = jb.h0 < 0 && jb.h0 > -sp.max_sc;
-                const bool outside = !job_in_planes(jb, d.n_bases);
+                const bool bad = (jb.h0 < 0 && jb.h0 > -sp.max_sc) || !job_in_planes(jb, d.n_bases);
+                const bool too_long = c.qlen > d.qmax || c.tlen > d.tmax || c.qlen > 65534 || !band_fits(c, sp.max_sc, W);
                 if (d.split && band_window(c.w, c.qlen, c.h0, sp.max_sc) != W) {
                     // another kernel's
-                } else if (bad_h0 || outside || c.qlen > d.qmax || c.tlen > d.tmax || c.qlen > 65534 ||
-                           !band_fits(c, sp.max_sc, W)) {
-                    if (r == 0) refuse(d, job, bad_h0 || outside ? G3X_ERR_INVALID : G3X_ERR_TOO_LONG);
-                } else if (c.tlen == 0) {
-                    if (r == 0) {
-                        refuse(d, job, G3X_OK);
-                        d.out[job] = g3x_ext_t{c.h0, 0, 0, 0, -1, 0};
-                    }
-                } else if (c.w < 0) {
-                    if (r == 0) finish_empty_band(d, job, c);
+                } else if (bad || too_long || c.tlen == 0 || c.w < 0) {
+                    if (r == 0) finish_unrun(d, job, c, bad ? G3X_ERR_INVALID : too_long ? G3X_ERR_TOO_LONG : G3X_OK);
                 } else {
                     J.job = job;
                     J.c = c;

@@ -175,7 +175,7 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                 if (lane == 0) first = atomicAdd(queue, __popc(want));
                 first = __shfl_sync(kAll, first, 0);
                 exhausted = first + __popc(want) >= n;
-                waves += first < n;
+                ++waves;
                 const int slot = first + __popc(want & ((1u << gb) - 1u));
                 bool fresh = false;
                 if (J.job < 0 && slot < n) {
@@ -191,17 +191,9 @@ __device__ __forceinline__ void run_groups(const LaunchDesc& d, const ScoreParam
                     const bool outside = !job_in_planes(jb, d.n_bases);
                     if (!fits && misfit) {
                         if (r == 0) misfit[atomicAdd(misfits, 1)] = job;
-                    } else if (too_long || outside || c.tlen == 0) {
-                        // refused before any base is read, or no rows: the initial results
-                        if (r == 0) {
-                            d.out[job] = too_long || outside ? g3x_ext_t{0, 0, 0, 0, 0, 0}
-                                                             : g3x_ext_t{c.h0, 0, 0, 0, -1, 0};
-                            d.status[job] = too_long ? G3X_ERR_TOO_LONG : outside ? G3X_ERR_INVALID : G3X_OK;
-                            if (d.cells) d.cells[job] = 0;
-                            if (d.rows) d.rows[job] = 0;
-                        }
-                    } else if (c.w < 0) {
-                        if (r == 0) finish_empty_band(d, job, c);
+                    } else if (too_long || outside || c.tlen == 0 || c.w < 0) {
+                        // refused before any base is read, or no cells
+                        if (r == 0) finish_unrun(d, job, c, too_long ? G3X_ERR_TOO_LONG : outside ? G3X_ERR_INVALID : G3X_OK);
                     } else {
                         fresh = true;
                         J.job = job;

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(128) rowpar_kernel(LaunchDesc d, ScoreParams s
         __syncwarp();
     }
     if (d.stats && r == 0) {
-        // (nothing from the groups without a job: see add_warp_stats)
+        // (no zeros: see add_warp_stats)
         if (busy_rows) atomicAdd(d.stats + 0, busy_rows);
         if (idle_rows) atomicAdd(d.stats + 1, idle_rows);
         if (gw == 0 && batches) atomicAdd(d.stats + 2, batches);

@@ -249,15 +249,16 @@ __device__ bool stage_job(int job, const LaunchDesc& d, const ScoreParams& sp,
     return true;
 }
 
-// A band below 0, which the clamp of ksw.cu:321-329 keeps, has no cell: row 0 begins at column -w, is
-// empty and ends the job, with a to-end score of 0 if that column is the query's end (ksw.cu:338-345,
-// 372-376).  For kernels whose rows take the band's first column from the row itself.
-__device__ __forceinline__ void finish_empty_band(const LaunchDesc& d, int job, const JobConst& c) {
-    const bool ends = c.qlen == -(int64_t)c.w;
-    d.out[job] = g3x_ext_t{c.h0, 0, 0, ends ? 1 : 0, ends ? 0 : -1, 0};
-    d.status[job] = G3X_OK;
+// Results of a job that is refused (status) or has no cells: no rows, or a band below 0, which the clamp
+// of ksw.cu:321-329 keeps: row 0 begins at column -w, is empty and ends the job, with a to-end score of 0
+// if that column is the query's end (ksw.cu:338-345, 372-376).  For kernels whose rows take the band's
+// first column from the row itself.
+__device__ __forceinline__ void finish_unrun(const LaunchDesc& d, int job, const JobConst& c, int32_t status) {
+    const bool ok = status == G3X_OK, row = ok && c.tlen > 0, ends = row && c.qlen + c.w == 0;
+    d.out[job] = g3x_ext_t{ok ? c.h0 : 0, 0, 0, ends ? 1 : 0, ok && !ends ? -1 : 0, 0};
+    d.status[job] = status;
     if (d.cells) d.cells[job] = 0;
-    if (d.rows) d.rows[job] = 1;
+    if (d.rows) d.rows[job] = row ? 1 : 0;
 }
 
 // Programmatic dependent launch in the width-class kernels.  pdl_trigger, first thing in the
@@ -281,8 +282,7 @@ __device__ __forceinline__ void add_warp_stats(unsigned long long* stats, unsign
         busy += __shfl_xor_sync(0xFFFFFFFFu, busy, o);
         idle += __shfl_xor_sync(0xFFFFFFFFu, idle, o);
     }
-    // (a warp that ran no job adds nothing: a class without jobs has thousands of those, and their adds to
-    // one address take 5 us)
+    // (no zeros: a class without jobs has thousands of warps, and their adds to one address take 5 us)
     const unsigned long long v = lane == 0 ? busy : lane == 1 ? idle : waves;
     if (lane < 3 && v) atomicAdd(stats + lane, v);
 }
