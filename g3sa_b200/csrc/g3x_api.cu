@@ -88,7 +88,7 @@ int batch_proto(const g3x_batch_opts_t* opts, int32_t* queue, LaunchDesc* d) {
                 : opts->kernel == G3X_KERNEL_LANE16 ? kKernelLane16
                 : opts->kernel == G3X_KERNEL_LANE2 ? kKernelLane2 : kKernelBand;
     if (d->kernel == kKernelBand) {
-        // one job per warp; tile carries the window (256, 512 or 1024 columns, 0 = 1024)
+        // 8-32 lanes per job; tile carries the window (256, 512 or 1024 columns, 0 = 1024)
         const int win = opts->tile ? opts->tile : 1024;
         if (win != 256 && win != 512 && win != 1024) return G3X_ERR_INVALID;
         d->lanes = 32; d->tile = win; d->persistent = plain ? 0 : 1; d->warps_per_block = 4;
@@ -192,7 +192,7 @@ static ClassRes ctx_res(g3x_ctx* ctx) {
 // The jobs of an unbounded last class (d: their order and count, on the row-parallel kernel's
 // settings).  Queries beyond the lane classes run in the band kernel where a window holds their
 // band: 1,500 segments of 500-5,000 bases at w = 500 take 32.8 ms row-parallel, which sweeps the row in
-// shared memory tile by tile, and 7.5 ms with the band's row in registers; 20,000 at w = 100 162 and
+// shared memory tile by tile, and 6.4 ms with the band's row in registers; 20,000 at w = 100 162 and
 // 8.1.  Shorter ones are here only for their scores, a few jobs not worth three launches.  queue:
 // four zeroed counters.
 static int launch_last(const LaunchDesc& d, const ScoreParams& sp, int32_t* queue, cudaStream_t st) {
@@ -769,7 +769,7 @@ int g3x_autotune_schedule(g3x_ctx* ctx, int32_t schedule, const g3x_score_t* sco
         if (!last && ring > 0 && ring < g3x::class_qcap(ctx->tiles, k, max_qlen) + 19 &&
             g3x::lane_ring_smem_per_warp(ring) <= 200 * 1024)
             for (int rf : {1, 8, 32}) cands[nc++] = Cand{1, ring, 0, rf};
-        // the band kernel (one warp per job), with the narrowest window that holds every band
+        // the band kernel (8-32 lanes per job), with the narrowest window that holds every band
         if (!last && wmax > 0 && 2 * wmax + 2 <= 1024) {
             const int win = 2 * wmax + 2 <= 256 ? 256 : 2 * wmax + 2 <= 512 ? 512 : 1024;
             cands[nc++] = Cand{32, win, 0, 1};

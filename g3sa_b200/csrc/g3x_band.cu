@@ -36,7 +36,7 @@
 // What bounds it: the integer ALU pipe, about 11 instructions per column and row beside 3
 // multiply-adds, and about 100 per row of a warp, whatever its groups.  The form that kept eh[] at its
 // own index, one warp per job and every edge in per-column selects took 34 a column: 20,000
-// segments of 500-5,000 bases at w = 100 21.5 ms, now 8.4 (870 GCUPS); 1,500 at w = 500 7.5 ms.
+// segments of 500-5,000 bases at w = 100 21.5 ms, now 8.2 (895 GCUPS); 1,500 at w = 500 6.4 ms.
 #include <cuda_runtime.h>
 #include "g3x_core.h"
 #include "g3x_group.cuh"
@@ -362,7 +362,9 @@ __global__ void __launch_bounds__(64) band_kernel(LaunchDesc d, ScoreParams sp) 
         const unsigned have = __ballot_sync(kAll, J.job >= 0) & leaders;
         if (!have) continue;
         jobs_run += __popc(have);
-        // the narrowest registers that hold the warp's bands: a row costs about 11 instructions a column
+        // the narrowest registers that hold the warp's bands: a row costs about 11 instructions a column.
+        // 224 is there for w = 100, BWA's default: 20k segments 8.2 ms, in 256 columns 8.9.  (192 beside it
+        // measured 7.3 against 8.1 for 20k at w = 90 and 4.0 against 4.4 for 3,000, where 256 takes 3.9.)
         const int cols = 2 * __reduce_max_sync(kAll, J.c.w) + 1;
 #define G3X_BAND(R) run_band<G, (R), kSym>(d, sp, J, pools, lane, rows_run)
         if constexpr (W == 256) {

@@ -142,7 +142,7 @@ constexpr int32_t kKernelRowpar = 2;    // one row per step, columns on lanes
 constexpr int32_t kKernelLane = 3;      // one job per lane
 constexpr int32_t kKernelLane16 = 4;    // one job per lane, int16x2 pair-column blocks
 constexpr int32_t kKernelLane2 = 5;     // one job per lane, two rows in flight
-constexpr int32_t kKernelBand = 6;      // one job per warp, the band's row buffer in registers
+constexpr int32_t kKernelBand = 6;      // 8-32 lanes per job, the band's row buffer in registers
 
 int launch_extend(const LaunchDesc& d, const ScoreParams& sp, cudaStream_t stream);
 

@@ -212,7 +212,7 @@ __device__ __forceinline__ void seg_steps(const SwDesc& d, const uint2 pool, con
 }
 
 // The row loop of one pass over registers H, E (slot MAXSEG - slen + j = segment j), over the last V
-// slots: every live quad of the warp has V - 3 .. V segments, so only the first four slots ask
+// slots: every live quad of the warp has V - 3 .. V segments, so only the first three slots ask
 // whether they are the quad's (a slot before its first segment holds zeros: score 0, no H, E or F),
 // and the others are straight code.  (One jump per row to a first slot common to the warp, and a guard
 // in every slot where there was none, took 390 instructions a row of 12 segments.)  A quad that is
