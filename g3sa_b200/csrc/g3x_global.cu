@@ -224,6 +224,15 @@ __global__ void __launch_bounds__(64) global_kernel(GlobalDesc d, ScoreParams sp
 // there on the sorted form's time hardly moves with the count, the direct one's grows with it.
 constexpr int kDirectPairs = 1024;
 
+// Large batches of very short pairs stay in the lane kernel, which has 32 of them a warp where the groups
+// have sixteen at most and one lane of each walks the CIGAR and MD.  Lane kernel and groups, us: up to 8
+// bases 100k pairs with MD 86 and 86, 130k 91 and 97, 190k 103 and 123, without 91 and 103; 12 bases 160k
+// with MD 130 and 133, 190k 133 and 153, without 114 and 119; 16 bases 190k with MD 163 and 177, without 141
+// and 134; 20 bases 160k 193 and 192, 190k 203 and 216; 23 bases 190k 240 and 239.
+static bool short_pairs(int qmax, bool md, int64_t n) {
+    return qmax <= (md ? 20 : 12) && n > (qmax <= 8 ? 114688 : 163840);
+}
+
 }  // namespace
 
 }  // namespace g3x
@@ -268,15 +277,19 @@ extern "C" int g3x_ksw_global2_batch(g3x_ctx* ctx, const g3x_score_t* score, con
     if (warp_smem > max_smem) return G3X_ERR_TOO_LONG;
     // The group kernel takes the jobs that fit it; the lane kernel is launched when there may be
     // others: values beyond int16, or bands beyond the widest group (a band is cut to the longer
-    // sequence).
-    const bool groups = c16, lanes = !c16 || std::min(max_w, std::max(d.qmax, d.tmax)) > kGlobalGroupMaxW;
+    // sequence).  may: which of them calls of these bounds launch at some number of pairs.
+    const bool brief = short_pairs(d.qmax, d_nm != nullptr, n), may_brief = short_pairs(d.qmax, d_nm != nullptr, 0x7FFFFFFF);
+    const bool groups = c16 && !brief;
+    const bool lanes = !groups || std::min(max_w, std::max(d.qmax, d.tmax)) > kGlobalGroupMaxW;
+    const bool may_groups = c16, may_lanes = lanes || may_brief;
     const int64_t cap = (int64_t)8 << 30;
     int wpb = 0, blocks = 0, gblocks = 0;
     int64_t need = 0;
     const int64_t zlane = (int64_t)d.tmax * d.ncol * 32, zgroup = global16_warp_bytes(d.tmax);
     // scratch: the resident warps' directions, at most 8 GiB; the two kernels run one after the
-    // other and share it
-    if (lanes) {
+    // other and share it.  It is sized by the bounds alone, for the whole device and whatever n is: a call
+    // captured after a smaller one of the same bounds must find its scratch.
+    if (may_lanes) {
         wpb = 2 * warp_smem <= max_smem ? 2 : 1;
         const int per_sm = resident_blocks(kern, 32 * wpb, wpb * warp_smem);
         blocks = sm_count() * std::max(per_sm, 1);
@@ -284,9 +297,7 @@ extern "C" int g3x_ksw_global2_batch(g3x_ctx* ctx, const g3x_score_t* score, con
         need = (int64_t)blocks * wpb * zlane;
     }
     const bool direct = groups && !lanes && n <= kDirectPairs;
-    if (groups) {
-        // (for the whole device whatever n is: a call captured after a smaller one within the same bounds
-        // must find its scratch)
+    if (may_groups) {
         gblocks = global16_blocks();
         while (gblocks > 1 && (int64_t)gblocks * kGlobal16Warps * zgroup > cap) gblocks = gblocks / 2;
         need = std::max(need, (int64_t)gblocks * kGlobal16Warps * zgroup);

@@ -230,6 +230,41 @@ def test_gpu_global_writes_every_refused_pair(n, mq, mt, mw):
     np.testing.assert_array_equal(n_cigar[~bad], n1)
 
 
+@pytest.mark.parametrize("max_len,n,md", [(9, 114688, True), (9, 114689, True), (21, 163841, True), (21, 163841, False), (13, 163841, False)])
+def test_gpu_global_short_pairs(max_len, n, md):
+    """Large batches of very short pairs on both sides of the line from which the lane kernel runs them, in one
+    context whose scratch an ordinary batch of the same bounds sized first."""
+    import torch
+    sc = g.default_score()
+    cj, u8 = nat.global_jobs(3000, max_len, max_len=max_len, ws=(0, 3, 5, 20, 50))
+    stride, md_stride = int((cj["qlen"] + cj["tlen"]).max()) + 2, 128
+    s1, c1, n1, _ = nat.oracle_global(cj, u8, sc, stride)
+    nm1, md1 = nat.oracle_nm_md(cj, u8, c1, n1, md_stride)
+    codes, nmask = g.pack_planes(u8)
+    c = g.Context(0)
+    for m in (3000, n):
+        jobs = np.resize(gpu_jobs(cj), m)
+        out = [torch.full((m * k,), 77, dtype=torch.int32, device="cuda") for k in (1, stride, 1, 1, 1)]
+        d_md = torch.zeros(m * md_stride, dtype=torch.uint8, device="cuda")
+        c.global_batch(sc, to_dev(jobs), m, to_dev(codes), to_dev(nmask), int(cj["qlen"].max()), int(cj["tlen"].max()),
+                       50, out[0], out[1], stride, out[2], out[3], d_nm=out[4] if md else None, d_md=d_md if md else None,
+                       md_stride=md_stride if md else 0)
+        torch.cuda.synchronize()
+        score, cig, nc, status, nm = [t.cpu().numpy() for t in out]
+        assert (status == 0).all()
+        np.testing.assert_array_equal(score, np.resize(s1, m))
+        np.testing.assert_array_equal(nc, np.resize(n1, m))
+        used = np.arange(stride)[None, :] < np.resize(n1, m)[:, None]
+        want = np.where(used, np.resize(c1, (m, stride)), 77)
+        np.testing.assert_array_equal(cig.view(np.uint32).reshape(m, stride), want)
+        if md:
+            np.testing.assert_array_equal(nm, np.resize(nm1, m))
+            text = d_md.cpu().numpy().reshape(m, md_stride)
+            for k in range(0, m, 997):
+                assert bytes(text[k]).split(b"\0")[0].decode() == md1[k % len(md1)]
+    c.close()
+
+
 def test_gpu_global_captured_after_a_smaller_call():
     """Scratch depends on the call's bounds, not on its pairs (up to the 1,024 that a context's order
     scratch always holds): a call of the same bounds is captured into a graph after a smaller one, and
